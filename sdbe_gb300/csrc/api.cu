@@ -29,6 +29,11 @@ int fail(sdbe_resampler *h, int code, const std::string &msg) {
     return code;
 }
 
+int check_status(sdbe_resampler *h) {
+    if (!*reinterpret_cast<volatile int *>(h->tc_status_host)) return SDBE_OK;
+    return fail(h, SDBE_ERR_CUDA, "a transform timed out on its mbarrier wait");
+}
+
 cudaError_t timed_begin(sdbe_resampler *h, int kind, int64_t units, cudaStream_t st, size_t *slot) {
     *slot = SIZE_MAX;
     if (!h->prof) return cudaSuccess;
@@ -473,6 +478,8 @@ int fft_chain_multi(std::vector<CallPlan> &cs) {
     sdbe_resampler *h0 = cs[0].h;
     cudaStream_t st = cs[0].st;
     const int n = static_cast<int>(cs.size());
+    for (const auto &c : cs)
+        if (int rc = check_status(c.h)) return rc;
     std::vector<int64_t> b(static_cast<size_t>(n), 0);
     {
         SegsA A{};
@@ -635,6 +642,12 @@ int sdbe_create(const sdbe_config *cfg, sdbe_resampler **out) {
                 cudaEventCreateWithFlags(&sg.out_free, cudaEventDisableTiming) == cudaSuccess;
     if (!ev_ok) return bail(SDBE_ERR_CUDA, "event creation failed");
     if (build_twiddles(h->tw, &h->tw_storage) != cudaSuccess) return bail(SDBE_ERR_NOMEM, "twiddle tables");
+    if (cudaHostAlloc(&h->tc_status_host, sizeof(int), cudaHostAllocMapped) != cudaSuccess)
+        return bail(SDBE_ERR_NOMEM, "cannot allocate the status flag");
+    *h->tc_status_host = 0;
+    if (cudaHostGetDevicePointer(reinterpret_cast<void **>(&h->tc_status), h->tc_status_host, 0) != cudaSuccess)
+        return bail(SDBE_ERR_CUDA, "status flag address");
+    h->tw.status = h->tc_status;
     bool ok = cudaMalloc(&h->spec, 2 * h->spec_pol_stride * sizeof(uint32_t)) == cudaSuccess &&
               cudaMalloc(&h->bitmap, static_cast<size_t>(cfg->max_frames) * 256) == cudaSuccess &&
               cudaMalloc(&h->counts, (static_cast<size_t>(cfg->max_frames) + 1) * sizeof(int32_t)) == cudaSuccess &&
@@ -948,6 +961,7 @@ int sdbe_swarm_c2r(sdbe_resampler *h, const uint32_t *spec, int64_t n_snapshots,
     if (unaligned(spec, 16) || unaligned(out, 16)) return fail(h, SDBE_ERR_ARG, "spectra and output must be 16-byte aligned");
     DeviceGuard g(h->cfg.device);
     if (h->cfg.precision != SDBE_PRECISION_FP32) return tc_swarm_c2r(h, spec, n_snapshots, out, pick(h, stream));
+    if (int rc = check_status(h)) return rc;
     SDBE_CK(h, launch_swarm_c2r(spec, 0, 0, n_snapshots, 1, out, 0, h->tw, pick(h, stream)));
     return SDBE_OK;
 }

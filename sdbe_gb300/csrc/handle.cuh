@@ -94,7 +94,7 @@ struct sdbe_resampler {
     int64_t tcf_half_bytes = 0;
     uint8_t *tcf_chain = nullptr; // tickets and stage counters of the one-launch waves (on first use)
     int64_t tcf_chain_bytes = 0;
-    int *tc_status_host = nullptr;  // 1 after a tensor-core barrier time-out (pinned, mapped)
+    int *tc_status_host = nullptr;  // 1 after a kernel's barrier wait timed out (pinned, mapped)
     int *tc_status = nullptr;       // its device address
     int64_t tc_test_timeout_ns = 0; // > 0: the next fast tensor-core launch withholds a signal (test hook)
     // Mar-2015 format: unpacked frames land here first; the last one is held
@@ -132,6 +132,9 @@ struct DeviceGuard {
         if (prev >= 0) cudaSetDevice(prev);
     }
 };
+
+// Whether an earlier call's kernel on this handle gave up on a barrier wait.
+int check_status(sdbe_resampler *h);
 
 #define SDBE_CK(h, call)                                                                             \
     do {                                                                                             \
@@ -273,6 +276,7 @@ int fft_chain(sdbe_resampler *h, const uint32_t *spec, int64_t spec_pol_stride, 
               const PayloadTarget &tgt, cudaStream_t st, OnWave on_wave) {
     int64_t b = 0;
     const bool win = h->cfg.threshold_mode == SDBE_THRESH_WINDOW;
+    if (int rc = check_status(h)) return rc;
     if (n_batches > 0 && !h->thresholds_set) {
         // First batch: floats + FP64 statistics, thresholds set once (.cu:953-986).
         SDBE_CK(h, launch_swarm_c2r(spec, spec_pol_stride, 0, kBatchSnaps, 2, h->ts, h->ts_pol_stride, h->tw, st));

@@ -7,7 +7,7 @@
 //   stage A  C2R 32768 per snapshot  = 16384-point complex inverse FFT plus
 //            Hermitian pre-processing, fed straight from the packed 2-bit
 //            spectrum (beng_int8_to_cufftComplex and the Nyquist memset fused);
-//            the next snapshot's 8 KB are prefetched with cp.async.
+//            the spectra of the next two snapshots are bulk-copied ahead.
 //   stage BC R2C 36608 per chunk = 18304-point complex FFT + post-processing,
 //            bins [skip, skip+16384] selected in registers, C2R 32768 through
 //            a 16384-point inverse FFT, then quantize2bit in the epilogue.
@@ -18,6 +18,7 @@
 #include "fft_core.cuh"
 #include "launchers.cuh"
 #include "sdbe_internal.cuh"
+#include "tcgen05.cuh"
 
 namespace sdbe {
 
@@ -28,7 +29,10 @@ constexpr int kNTB = 512;   // stage BC threads: 4 warps per SM sub-partition ->
 // distinct bank pairs (see fft18304_from_global); the 16384-point transforms
 // keep one per 32 (their layouts are built on it).
 __host__ __device__ constexpr int padb(int a) { return a + (a >> 4); }
-constexpr int kPadA = padded_len(kMA);
+// One of the 16 sub-transforms of the inverse 16384: 32 rows of 33 slots, and
+// one more so that 16 consecutive columns' stores land in 16 bank pairs.
+constexpr int kSub = 1057;
+constexpr int kPadA = 16 * kSub;
 constexpr int kPadB = padb(kMB) + 1;
 
 // Shared-memory twiddle tables (float2).  The per-pass tables are laid out
@@ -40,7 +44,7 @@ constexpr int kT13 = 12 * 16;          // W_208^{k r}, r = 1..12, k = 0..15   (1
 constexpr int kH18304 = tp_len(143);   // W_18304^{128 a}
 constexpr int kTwA = kT32 + 2 * kT128;               // stage A tables
 constexpr int kTwB = kTwA + kT13 + kH18304 + kT128;  // stage BC tables
-constexpr size_t kSmemA = 2 * kGroups * sizeof(uint32_t) + (kPadA + kTwA) * sizeof(float2);
+constexpr size_t kSmemA = 2 * kGroups * sizeof(uint32_t) + (24 * kSub + kTwA) * sizeof(float2);
 constexpr size_t kSmemB = (kPadB + kTwB) * sizeof(float2);
 // Stage BC fits the 164 KB shared-memory carveout (with its 512-byte static
 // reduction buffer and the 1 KB reserved per block).  Above it (184 KB: the
@@ -106,10 +110,8 @@ __constant__ uint8_t kFirstPassGroups[144] = {
 // ---------------------------------------------------------------------------
 // Inverse 16384-point FFT, radices 32 x 32 x 16 (Stockham).  zin(v) gives
 // input elements col + 512 r, r < 32, of this thread's first-pass column
-// `col` (a permutation of the thread index whose 16 values in each half-warp
-// are distinct mod 16; zin may read `sm`: a barrier separates those reads
-// from the writes); epi(jj, u) receives outputs z[jj + 1024 r], r < 16.
-// blockDim.x is 512.
+// `col` (a permutation of the thread index); epi(jj, u) receives outputs
+// z[jj + 1024 r], r < 16.  blockDim.x is 512.
 // The last pass's per-thread twiddle bases W_16384^(tid s), s = 1..3, and
 // W_16384^(4 tid a), a = 1..3: they depend on the thread only, so a
 // persistent kernel can form them once.
@@ -126,62 +128,67 @@ __device__ __forceinline__ LastTw last_tw(const TabsA &T) {
     return t;
 }
 
-// ZIN_SM: zin reads `sm`, so a barrier must separate those reads from the
-// first pass's stores.  A caller whose zin reads other memory, and whose
-// previous smem reads are behind a barrier already, passes false.
-template <bool ZIN_SM = true, class In, class Epi>
-__device__ __forceinline__ void ifft16384(float2 *sm, const TabsA &T, In zin, Epi epi, int col, const LastTw &lt) {
-    const int tid = threadIdx.x;
+// The transform is 16 transforms of 1024 points (first-pass columns col = w
+// mod 16, radices 32 x 32), each in its own kSub slots of `sm`, and a last
+// radix-16 pass across them.  Column w + 16 i leaves its 32 outputs in row i
+// of sub-transform w; the second pass, one warp per sub-transform, reads
+// column l of those rows (lane l) and writes its outputs to the very slots it
+// read, so no barrier separates its loads from its stores, and a warp that
+// takes its own sub-transform's columns needs no block barrier between the
+// first two passes at all.
+
+// First pass: the DFT-32 outputs v of column `col`, its sub-transform's slots at `slots`.
+__device__ __forceinline__ void inv_store1(float2 *slots, int col, const float2 *v) {
+    float2 *dst = slots + 33 * (col >> 4);
+#pragma unroll
+    for (int r = 0; r < 32; ++r) dst[r] = v[r];
+}
+
+// The second pass's twiddles W_1024^{l r} = A[r/8] * S[r%8] of lane l, r = 1..31 (w[0] unused).
+__device__ __forceinline__ void pass2_twiddles(const TabsA &T, float2 *w) {
+    const float2 *tj = T.t32 + (threadIdx.x & 31);
+    float2 S[8], A[4];
+#pragma unroll
+    for (int s = 1; s < 8; ++s) S[s] = tj[32 * (s - 1)];
+#pragma unroll
+    for (int a = 1; a < 4; ++a) A[a] = tj[32 * (6 + a)];
+    w[0] = make_float2(1.f, 0.f);
+#pragma unroll
+    for (int r = 1; r < 32; ++r) {
+        const int a = r >> 3, s = r & 7;
+        w[r] = a == 0 ? S[s] : (s == 0 ? A[a] : cmul(A[a], S[s]));
+    }
+}
+
+// Second pass of the sub-transform at `slots`, in place; apply(v) multiplies
+// v[r] by conj W_1024^{l r}.
+template <class Apply>
+__device__ __forceinline__ void inv_pass2(float2 *slots, Apply apply) {
     float2 v[32];
-    if (tid < 512) {
-        zin(v);
-        dft<32, true>(v);
-    }
-    if constexpr (ZIN_SM) __syncthreads();
-    // padded addresses as base + compile-time offsets: pad(32 t + r) = 33 t + r,
-    // pad(t + 512 r) = pad(t) + 528 r, pad(b + 32 r) = pad(b) + 33 r (b % 32 + r < 32 not
-    // needed: b is a multiple of 1024 plus a lane), pad(j + 1024 r) = pad(j) + 1056 r.
-    if (tid < 512) {
-        float2 *dst = sm + 33 * col;
+    float2 *p = slots + (threadIdx.x & 31);
 #pragma unroll
-        for (int r = 0; r < 32; ++r) dst[r] = v[r];
-    }
-    __syncthreads();
-    if (tid < 512) {
-        const float2 *src = sm + pad(tid);
+    for (int r = 0; r < 32; ++r) v[r] = p[33 * r];
+    apply(v);
+    dft<32, true>(v);
 #pragma unroll
-        for (int r = 0; r < 32; ++r) v[r] = src[528 * r];
-        // W_1024^{jm r} = A[r/8] * S[r%8]
-        const float2 *tj = T.t32 + (tid & 31);
-        float2 S[8], A[4];
-#pragma unroll
-        for (int s = 1; s < 8; ++s) S[s] = tj[32 * (s - 1)];
-#pragma unroll
-        for (int a = 1; a < 4; ++a) A[a] = tj[32 * (6 + a)];
-#pragma unroll
-        for (int r = 1; r < 32; ++r) {
-            const int a = r >> 3, s = r & 7;
-            const float2 w = a == 0 ? S[s] : (s == 0 ? A[a] : cmul(A[a], S[s]));
-            v[r] = cmulc(v[r], w);
-        }
-        dft<32, true>(v);
-    }
-    __syncthreads();
-    if (tid < 512) {
-        float2 *dst = sm + (tid >> 5) * 1056 + (tid & 31);
-#pragma unroll
-        for (int r = 0; r < 32; ++r) dst[33 * r] = v[r];
-    }
-    __syncthreads();
-    // last pass: jj = tid + 512 i, i = 0, 1; W_16384^(jj s) = W^(tid s) W^(512 i s)
+    for (int r = 0; r < 32; ++r) p[33 * r] = v[r];
+}
+
+// Last pass: jj = tid + 512 i, i = 0, 1; W_16384^(jj s) = W^(tid s) W^(512 i s).
+// at(r) is where sub-transform r's slots begin (r a compile-time index);
+// read_done() runs after this thread's last loads.
+template <class At, class Epi, class Done>
+__device__ __forceinline__ void inv_pass3(At at, const LastTw &lt, Epi epi, Done read_done) {
+    const int tid = threadIdx.x;
     const float2 *S0 = lt.S0, *A0 = lt.A0;
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
         const int jj = tid + 512 * i;
         float2 u[16];
-        const float2 *src = sm + pad(jj);
+        const int o = pad(jj);
 #pragma unroll
-        for (int r = 0; r < 16; ++r) u[r] = src[1056 * r];
+        for (int r = 0; r < 16; ++r) u[r] = at(r)[o];
+        if (i == 1) read_done();
         // W_16384^{jj r} = A[r/4] * S[r%4]
         float2 S[4], A[4];
         S[1] = i ? mul_tc<kMA, 512, false>(S0[1]) : S0[1];
@@ -201,98 +208,70 @@ __device__ __forceinline__ void ifft16384(float2 *sm, const TabsA &T, In zin, Ep
     }
 }
 
-// The same, forming the last pass's twiddle bases on each call (for kernels
-// with no registers to keep them across items).
-template <class In, class Epi>
-__device__ __forceinline__ void ifft16384(float2 *sm, const TabsA &T, In zin, Epi epi, int col = threadIdx.x) {
-    ifft16384(sm, T, zin, epi, col, last_tw(T));
-}
-
 // f(integral_constant<int, R>) for each R: a loop over compile-time indices.
 template <int... R, class F>
 __device__ __forceinline__ void for_r(std::integer_sequence<int, R...>, F f) {
     (f(std::integral_constant<int, R>{}), ...);
 }
 
-// Forward 18304-point FFT of z[m] = x[2m] + i x[2m+1] read from global memory;
-// result Z in natural order in `sm` (padded with padb).  In-place decimation
-// in time, radices 16 (from global) x 13 x 11 x 8: the first pass reads
-// z[j + 1144 r] (8 consecutive j per 8 lanes: 64-B segments) and writes its 16
-// outputs to slots 16*rho(j) + r, rho = digit reversal of j over (8, 11, 13);
-// every later butterfly reads and writes the same slots g*Ns*R + k + Ns*r
-// with twiddles W_{Ns*R}^{k r}, so passes need no staging.
-//
-// R2C: the last pass also applies the R2C pairing, leaving X[q] (q <= 18304,
+// Radix 13, Ns = 16: twiddles W_208^{k r}, k = 0..15, the same for every
+// butterfly of a thread that keeps its k; butterfly k of block b (208 slots).
+__device__ __forceinline__ void pass13_twiddles(const TabsB &T, int k, float2 *w13) {
+#pragma unroll
+    for (int r = 1; r < 13; ++r) w13[r] = T.t13[16 * (r - 1) + k];
+}
+__device__ __forceinline__ void fwd_pass13(float2 *sm, const float2 *w13, int b, int k) {
+    float2 *p = sm + padb(b * 208 + k);  // padb(base + 16 r) = padb(base) + 17 r
+    float2 v[13];
+#pragma unroll
+    for (int r = 0; r < 13; ++r) v[r] = p[17 * r];
+#pragma unroll
+    for (int r = 1; r < 13; ++r) v[r] = cmul(v[r], w13[r]);
+    dft<13, false>(v);
+#pragma unroll
+    for (int r = 0; r < 13; ++r) p[17 * r] = v[r];
+}
+
+// Radix 11, Ns = 208: twiddles W_2288^{k r}.  Butterfly (m, k) is at base
+// 2288 m + k, m < 8, k < 208; thread t takes k = t % 208 and m = t / 208
+// + j nk, nk = the threads sharing its k, so its ten twiddles are formed
+// once per transform, from the two-level W_18304 tables (at most 4
+// butterflies a thread, as with b = t + 512 j).
+__device__ __forceinline__ void fwd_pass11(float2 *sm, const TabsB &T) {
+    static_assert(kNTB == 512, "512 threads share 208 x 8 butterflies");
+    const int t = threadIdx.x, k = t % 208, nk = k < 512 - 2 * 208 ? 3 : 2;
+    float2 w11[11];
+#pragma unroll
+    for (int r = 1; r < 11; ++r) w11[r] = tw2(T.h18304, T.l18304, 8 * k * r);  // W_2288^(k r), 8 k r < 18304
+    for (int m = t / 208; m < 8; m += nk) {
+        float2 *p = sm + padb(2288 * m + k);  // padb(base + 208 r) = padb(base) + 221 r
+        float2 v[11];
+#pragma unroll
+        for (int r = 0; r < 11; ++r) v[r] = p[221 * r];
+#pragma unroll
+        for (int r = 1; r < 11; ++r) v[r] = cmul(v[r], w11[r]);
+        dft<11, false>(v);
+#pragma unroll
+        for (int r = 0; r < 11; ++r) p[221 * r] = v[r];
+    }
+}
+
+// Radix 8, Ns = 2288, the last pass: twiddles W_18304^{k r}.  With R2C it also applies the R2C pairing, leaving X[q] (q <= 18304,
 // X[18304] in the spare slot padb(18304)) instead of Z.  Its butterfly k
 // holds Z[k + 2288 r] and butterfly 2288 - k holds their mirrors Z[18304 - q]
 // at r' = 7 - r, so one thread takes both (k = 0 and k = 1144 are their own
 // mirrors) and pairs in registers: one pass and one barrier fewer.
+//
+// W_36608^(u + 2288 r) = wu W_16^r with its rounding pinned (MID: the unit u = 1144).
+template <int R, bool MID = false>
+__device__ __forceinline__ float2 r2c_tw(float2 wu) {
+    if constexpr (R == 0) return wu;
+    constexpr int X = MID ? (R == 3 ? 1 : 0) : (R >= 5 ? 2 : 0), Y = MID ? (R == 3 ? 0 : 1) : (R >= 5 ? 2 : 1);
+    return cmul_rn<X, Y>(wu, make_float2(TwC<16, R>::c, TwC<16, R>::s));
+}
 template <bool R2C>
-__device__ __forceinline__ void fft18304_from_global(float2 *sm, const float2 *__restrict__ z, const TabsB &T) {
-    constexpr int NB1 = kMB / 16;  // 1144 = 143 groups of 8
-    for (int h = threadIdx.x >> 4; h < 72; h += blockDim.x >> 4) {
-        const int g = kFirstPassGroups[2 * h + ((threadIdx.x >> 3) & 1)];
-        if (g == 255) continue;
-        const int c = threadIdx.x & 7, j = 8 * g + c;
-        float2 v[16];
-        // read-only loads (ld.global.nc), not streaming ones (ld.global.cs):
-        // measured 2% faster for the kernel, though L1 hits stay rare (7% of
-        // sectors), so the gain is not from reuse of the other half of each
-        // 128-byte line
-#pragma unroll
-        for (int r = 0; r < 16; ++r) v[r] = __ldg(z + j + NB1 * r);
-        dft<16, false>(v);
-        // rho(8g + c) = g/11 + 13 (g%11) + 143 c; padb(16 rho + r) = 17 rho + r (r < 16)
-        float2 *d = sm + 17 * (g / 11 + 13 * (g % 11) + 143 * c);
-#pragma unroll
-        for (int r = 0; r < 16; ++r) d[r] = v[r];
-    }
-    __syncthreads();
-    // radix 13, Ns = 16: twiddles W_208^{k r}; k = b & 15 = tid & 15 for all of a
-    // thread's butterflies (blockDim.x is a multiple of 16), so they load once
-    {
-        const int k = threadIdx.x & 15;
-        float2 w13[13];
-#pragma unroll
-        for (int r = 1; r < 13; ++r) w13[r] = T.t13[16 * (r - 1) + k];
-        for (int b = threadIdx.x; b < kMB / 13; b += blockDim.x) {
-            float2 *p = sm + padb((b >> 4) * 208 + k);  // padb(base + 16 r) = padb(base) + 17 r
-            float2 v[13];
-#pragma unroll
-            for (int r = 0; r < 13; ++r) v[r] = p[17 * r];
-#pragma unroll
-            for (int r = 1; r < 13; ++r) v[r] = cmul(v[r], w13[r]);
-            dft<13, false>(v);
-#pragma unroll
-            for (int r = 0; r < 13; ++r) p[17 * r] = v[r];
-        }
-    }
-    __syncthreads();
-    // radix 11, Ns = 208: twiddles W_2288^{k r}.  Butterfly (m, k) is at base
-    // 2288 m + k, m < 8, k < 208; thread t takes k = t % 208 and m = t / 208
-    // + j nk, nk = the threads sharing its k, so its ten twiddles are formed
-    // once per transform, from the two-level W_18304 tables (at most 4
-    // butterflies a thread, as with b = t + 512 j).
-    {
-        static_assert(kNTB == 512, "512 threads share 208 x 8 butterflies");
-        const int t = threadIdx.x, k = t % 208, nk = k < 512 - 2 * 208 ? 3 : 2;
-        float2 w11[11];
-#pragma unroll
-        for (int r = 1; r < 11; ++r) w11[r] = tw2(T.h18304, T.l18304, 8 * k * r);  // W_2288^(k r), 8 k r < 18304
-        for (int m = t / 208; m < 8; m += nk) {
-            float2 *p = sm + padb(2288 * m + k);  // padb(base + 208 r) = padb(base) + 221 r
-            float2 v[11];
-#pragma unroll
-            for (int r = 0; r < 11; ++r) v[r] = p[221 * r];
-#pragma unroll
-            for (int r = 1; r < 11; ++r) v[r] = cmul(v[r], w11[r]);
-            dft<11, false>(v);
-#pragma unroll
-            for (int r = 0; r < 11; ++r) p[221 * r] = v[r];
-        }
-    }
-    __syncthreads();
-    // radix 8, Ns = 2288: twiddles W_18304^{k r} = A[r/4] * S[r%4]
+__device__ __forceinline__ void fwd_pass8(float2 *sm, const TabsB &T) {
+    // twiddles W_18304^{k r} = A[r/4] * S[r%4]
     // butterfly k with its twiddles S[q] = W^(k q), q = 1..3, and A1 = W^(4 k)
     auto bfly8w = [&](int k, float2 *v, const float2 *S, float2 A1) {
         const float2 *p = sm + padb(k);  // padb(k + 2288 r) = padb(k) + 2431 r
@@ -358,7 +337,7 @@ __device__ __forceinline__ void fft18304_from_global(float2 *sm, const float2 *_
                 for_r(std::make_integer_sequence<int, 4>{}, [&](auto rc) {
                     constexpr int r = decltype(rc)::value;
                     float2 xq, xmq;
-                    r2c_pair(a[r], a[7 - r], mul_tc<16, r, false>(wu), xq, xmq);
+                    r2c_pair(a[r], a[7 - r], r2c_tw<r, true>(wu), xq, xmq);
                     pa[2431 * r] = xq;
                     pa[2431 * (7 - r)] = xmq;
                 });
@@ -373,13 +352,53 @@ __device__ __forceinline__ void fft18304_from_global(float2 *sm, const float2 *_
                 for_r(std::make_integer_sequence<int, 8>{}, [&](auto rc) {
                     constexpr int r = decltype(rc)::value;
                     float2 xq, xmq;
-                    r2c_pair(a[r], b[7 - r], mul_tc<16, r, false>(wu), xq, xmq);
+                    r2c_pair(a[r], b[7 - r], r2c_tw<r>(wu), xq, xmq);
                     pa[2431 * r] = xq;
                     pb[2431 * (7 - r)] = xmq;
                 });
             }
         });
     }
+}
+
+// Forward 18304-point FFT of z[m] = x[2m] + i x[2m+1] read from global memory;
+// result Z in natural order in `sm` (padded with padb).  In-place decimation
+// in time, radices 16 (from global) x 13 x 11 x 8: the first pass reads
+// z[j + 1144 r] (8 consecutive j per 8 lanes: 64-B segments) and writes its 16
+// outputs to slots 16*rho(j) + r, rho = digit reversal of j over (8, 11, 13);
+// every later butterfly reads and writes the same slots g*Ns*R + k + Ns*r
+// with twiddles W_{Ns*R}^{k r}, so passes need no staging.
+//
+__device__ __forceinline__ void fft18304_from_global(float2 *sm, const float2 *__restrict__ z, const TabsB &T) {
+    constexpr int NB1 = kMB / 16;  // 1144 = 143 groups of 8
+    for (int h = threadIdx.x >> 4; h < 72; h += blockDim.x >> 4) {
+        const int g = kFirstPassGroups[2 * h + ((threadIdx.x >> 3) & 1)];
+        if (g == 255) continue;
+        const int c = threadIdx.x & 7, j = 8 * g + c;
+        float2 v[16];
+        // read-only loads (ld.global.nc), not streaming ones (ld.global.cs):
+        // measured 2% faster for the kernel, though L1 hits stay rare (7% of
+        // sectors), so the gain is not from reuse of the other half of each
+        // 128-byte line
+#pragma unroll
+        for (int r = 0; r < 16; ++r) v[r] = __ldg(z + j + NB1 * r);
+        dft<16, false>(v);
+        // rho(8g + c) = g/11 + 13 (g%11) + 143 c; padb(16 rho + r) = 17 rho + r (r < 16)
+        float2 *d = sm + 17 * (g / 11 + 13 * (g % 11) + 143 * c);
+#pragma unroll
+        for (int r = 0; r < 16; ++r) d[r] = v[r];
+    }
+    __syncthreads();
+    {
+        const int k = threadIdx.x & 15;
+        float2 w13[13];
+        pass13_twiddles(T, k, w13);
+        for (int b = threadIdx.x; b < kMB / 13; b += blockDim.x) fwd_pass13(sm, w13, b >> 4, k);
+    }
+    __syncthreads();
+    fwd_pass11(sm, T);
+    __syncthreads();
+    fwd_pass8<false>(sm, T);
     __syncthreads();
 }
 
@@ -399,14 +418,22 @@ __device__ __forceinline__ float2 r2c_bin(const float2 *sm, int q, float2 w) {
 // Hermitian pre-processing of a C2R of length 32768 from bins Y[0..16384],
 // given we = e^{+2 pi i k/32768}:
 //   Z[k] = (Y[k] + conj Y[M-k]) + i we (Y[k] - conj Y[M-k]),
-// imaginary parts of Y[0] and Y[16384] ignored (as cuFFT / numpy do).
+// imaginary parts of Y[0] and Y[16384] ignored (as cuFFT / numpy do).  X, Y:
+// the product's rounding (cmul_rn), X < 0 leaves it to the compiler.
+template <int X = -1, int Y = -1>
 __device__ __forceinline__ float2 c2r_pre(float2 y, float2 ym, int k, float2 we) {
     if (k == 0) {
         y.y = 0.f;
         ym.y = 0.f;
     }
     const float2 e = make_float2(y.x + ym.x, y.y - ym.y);
-    const float2 o = cmul(make_float2(y.x - ym.x, y.y + ym.y), we);
+    const float2 d = make_float2(y.x - ym.x, y.y + ym.y);
+    float2 o;
+    if constexpr (X < 0) {
+        o = cmul(d, we);
+    } else {
+        o = cmul_rn<X, Y>(d, we);
+    }
     return make_float2(e.x - o.y, e.y + o.x);
 }
 
@@ -416,14 +443,41 @@ __device__ __forceinline__ float2 c2r_tw(float2 base) {
     return mul_tc<64, R, true>(base);
 }
 
-// First-pass column of thread t for the paired C2R input below: lanes l < 16
-// of warp w take b = 16 w + l, lanes l >= 16 take 512 - (16 w + l - 16), so
-// lanes l and l ^ 16 hold mirror columns (b + b' = 512); warp 0's lane 16
-// takes 256.  The 16 columns of each half-warp are distinct mod 16.
+// The same with each product's rounding pinned, for stage BC.
+template <int R>
+__device__ __forceinline__ float2 c2r_tw_rn(float2 base) {
+    if constexpr (R == 0) return base;
+    constexpr bool both = R == 1 || (R >= 7 && R <= 9) || R == 15;
+    constexpr int X = both || R <= 6 ? (R <= 15 ? 2 : 0) : 0;
+    constexpr int Y = both || (R >= 10 && R <= 14) ? 2 : ((R >= 17 && R <= 25) || R == 31 ? 1 : 0);
+    return cmul_rn<X, Y>(base, make_float2(TwC<64, R>::c, -TwC<64, R>::s));
+}
+
+// First-pass columns for the paired C2R input below, numbered so that slots
+// l and l ^ 16 hold mirror columns (b + b' = 512); slot 16 takes 256.
 __device__ __forceinline__ int c2r_col(int t) {
     const int w = t >> 5, l = t & 31;
     if (l < 16) return 16 * w + l;
     return (w == 0 && l == 16) ? 256 : 512 - 16 * w - (l - 16);
+}
+// The slot of c2r_col that thread t takes.  Columns w + 16 i and their mirrors
+// 512 - w - 16 i = (16 - w) + 16 (31 - i) belong to sub-transforms w and
+// 16 - w, so two warps take both between them: warps 2w and 2w + 1 the halves
+// i < 16 and i >= 16 of sub-transform w in lanes l < 16 and the mirrors in
+// lanes l ^ 16 (w = 1..7); then warp 2w runs the second pass of sub-transform
+// w, warp 2w + 1 of 16 - w, and only the two of them wait for each other.
+// Sub-transforms 0 and 8 are their own mirrors: warps 0 and 1 (warp 0's lane
+// 16 takes column 256, the other column, besides lane 0's column 0, that is
+// its own mirror).
+__device__ __forceinline__ int c2r_slot(int t) {
+    const int w = t >> 6, s = (t >> 5) & 1, l = t & 31;
+    const int b = (w == 0 ? 8 * s : w + 256 * s) + 16 * (l & 15);  // column of lane l & 15
+    const int lo = b < 256 ? b : 512 - b;
+    return 32 * (lo >> 4) + (lo & 15) + 16 * ((l >> 4) ^ (b > 256 ? 1 : 0));
+}
+__device__ __forceinline__ int c2r_sub(int t) {
+    const int w = t >> 6, s = (t >> 5) & 1;
+    return w == 0 ? 8 * s : (s ? 16 - w : w);
 }
 
 // The C2R 32768 input Z[col + 512 r], r < 32, from the bins Y[0..16384]
@@ -435,55 +489,39 @@ __device__ __forceinline__ int c2r_col(int t) {
 // and 256 are their own mirrors (M - 512 p = 512 (32 - p); M - 256 - 512 p
 // = 256 + 512 (31 - p)) and keep both halves; column 0 forms Z[8192] alone.
 // lo(p) = Y[col + 512 p] (p <= 16), hi(p) = Y[M - col - 512 p] (p < 16);
-// wcol = e^{2 pi i col/32768}.
+// we[p] = e^{2 pi i (col + 512 p)/32768}, w16 its value at p = 16.
 template <bool NYQ_ZERO, class Lo, class Hi>
-__device__ __forceinline__ void c2r_paired(float2 *v, int col, float2 wcol, Lo lo, Hi hi) {
+__device__ __forceinline__ void c2r_paired(float2 *v, int col, const float2 *we, float2 w16, Lo lo, Hi hi) {
     const int lane = threadIdx.x & 31;
-    auto pairs = [&](auto w0c) {
-        constexpr bool W0 = decltype(w0c)::value;
-        for_r(std::make_integer_sequence<int, 16>{}, [&](auto pc) {
-            constexpr int p = decltype(pc)::value;
-            float2 y = lo(pc), ym = hi(pc);
-            if (W0 && p == 0 && col == 0) {
-                y.y = 0.f;
-                ym = NYQ_ZERO ? make_float2(0.f, 0.f) : make_float2(ym.x, 0.f);
-            }
-            float2 zk, zmk;
-            c2r_pair(y, ym, c2r_tw<p>(wcol), zk, zmk);
-            v[p] = zk;
-            const float2 x = make_float2(__shfl_xor_sync(0xffffffffu, zmk.x, 16), __shfl_xor_sync(0xffffffffu, zmk.y, 16));
-            if constexpr (!W0) {
-                v[31 - p] = x;
-            } else {  // selects, not branches: warp 0 must not fall behind
-                const bool own = lane == 16;
-                v[31 - p] = make_float2(own ? zmk.x : x.x, own ? zmk.y : x.y);
-                if constexpr (p >= 1) {
-                    const bool c0 = lane == 0;
-                    v[32 - p] = make_float2(c0 ? zmk.x : v[32 - p].x, c0 ? zmk.y : v[32 - p].y);
-                }
-            }
-        });
-    };
-    if (threadIdx.x >= 32) {
-        pairs(std::false_type{});
-    } else {
-        pairs(std::true_type{});
+    // Every warp runs the same code (a second copy for warp 0 would be fetched
+    // beside the others').  Lane 16 of warp 0 (column 256) keeps its own mirror
+    // halves; lane 0 (column 0) its own too, one element on.
+    const bool w0 = threadIdx.x < 32, c0 = threadIdx.x == 0;
+    const int src = w0 && lane == 16 ? lane : lane ^ 16;
+    for_r(std::make_integer_sequence<int, 16>{}, [&](auto pc) {
+        constexpr int p = decltype(pc)::value;
+        float2 y = lo(pc), ym = hi(pc);
+        if (p == 0 && col == 0) {
+            y.y = 0.f;
+            ym = NYQ_ZERO ? make_float2(0.f, 0.f) : make_float2(ym.x, 0.f);
+        }
+        float2 zk, zmk;
+        c2r_pair_rn<p == 0 ? 1 : 0, 1>(y, ym, we[p], zk, zmk);
+        v[p] = zk;
+        v[31 - p] = make_float2(__shfl_sync(0xffffffffu, zmk.x, src), __shfl_sync(0xffffffffu, zmk.y, src));
+        if constexpr (p >= 1) v[32 - p] = make_float2(c0 ? zmk.x : v[32 - p].x, c0 ? zmk.y : v[32 - p].y);
+    });
+    if (w0) {
         // column 0: Z[8192] = Y[8192] + conj Y[8192] + i e^{i pi/2} (Y[8192] - conj Y[8192]);
         // the other lanes' lo(16) is in range and discarded
         const float2 y = lo(std::integral_constant<int, 16>{});
-        const float2 z = c2r_pre(y, y, 8192, c2r_tw<16>(wcol));
-        const bool c0 = lane == 0;
+        const float2 z = c2r_pre(y, y, 8192, w16);
         v[16] = make_float2(c0 ? z.x : v[16].x, c0 ? z.y : v[16].y);
     }
 }
 
-
-__device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
-    const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_1() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
+// Barrier `id` (1..15; 0 is __syncthreads) of n threads.
+__device__ __forceinline__ void bar_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
 
 // ---------------------------------------------------------------------------
 // Stage A (persistent): items = n_snaps x n_pols.  Packed spectrum of snapshot
@@ -496,58 +534,160 @@ __device__ __forceinline__ int seg_of(const Segs &S, int64_t item) {
     return j;
 }
 
+// The stage-A pipeline of one CTA.  A warp's work on an item is its input
+// columns (pairing and DFT-32), the first two passes of one sub-transform and
+// its share of the last pass.  Only the last pass needs every warp's earlier
+// work, and only the first pass's stores overwrite what every warp has read,
+// so each of these two dependencies is an mbarrier (one arrival per warp) with
+// other work between the arrival and the wait: a warp that has finished its
+// second pass forms the NEXT item's input columns before it waits for the
+// others, parking the 64 registers in tensor memory.  In a plain barrier
+// form, warps that ran in step competed for the shared-memory pipe in one
+// phase and for the FMA pipe in the next, and each was idle a third of the
+// time.
+struct PipeA {
+    uint64_t full[2];  // spectrum of an even / odd item landed
+    uint64_t read;     // a warp's last-pass loads are done
+    uint64_t second;   // a warp's second pass is stored
+    uint32_t tmem;
+    int err;
+};
+// Tensor memory columns: parked registers, 64 for each of the four warps of a
+// lane quarter, and the second pass's twiddles, 64, the same for the four
+// (forming them anew costs 84 instructions and 10 loads a thread and item).
+constexpr uint32_t kColPark = 0, kColTw2 = 256, kColsA = 512;
+
+// Shared memory holds the sub-transforms of an item and a half: three blocks
+// of eight, item k in blocks 2k and 2k + 1 (mod 3).  Its first block is never
+// one that item k - 1 is still read from, so the eight warps whose columns go
+// there (warps 0-7: sub-transforms 0, 8, 1, 15, 2, 14, 3, 13) store without
+// waiting, half an item ahead of the other eight: one half's shared-memory
+// phases meet the other half's arithmetic.
+constexpr int kBlkA = 8 * kSub;
+__host__ __device__ constexpr bool blk_second(int sub) { return (sub >= 4 && sub <= 7) || (sub >= 9 && sub <= 12); }
+__host__ __device__ constexpr int blk_index(int sub) {  // warps 2 p and 2 p + 1 hold sub-transforms p and 16 - p
+    const int p = sub == 8 ? 0 : (sub > 8 ? 16 - sub : sub);
+    return 2 * (p & 3) + (sub >= 8 ? 1 : 0);
+}
+
 __global__ void __launch_bounds__(kNTA, 1) k_swarm_c2r(const __grid_constant__ SegsA S, Twiddles tw) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     uint32_t *sp = reinterpret_cast<uint32_t *>(smem_raw);  // [2][2048] double buffer
     float2 *sm = reinterpret_cast<float2 *>(smem_raw + 2 * kGroups * sizeof(uint32_t));
-    TabsA T = tabs_a_at(sm + kPadA);
+    __shared__ PipeA P;
+    TabsA T = tabs_a_at(sm + 3 * kBlkA);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        tc5::mbar_init(&P.full[0], 1);
+        tc5::mbar_init(&P.full[1], 1);
+        tc5::mbar_init(&P.read, kNTA / 32);
+        tc5::mbar_init(&P.second, kNTA / 32);
+        tc5::fence_mbar_init();
+        P.err = 0;
+    }
+    if (warp == 0) tc5::tmem_alloc(&P.tmem, kColsA);
     load_tabs_a(T, tw);
-    const int col = c2r_col(threadIdx.x);               // the inverse's first-pass column
+    const int col = c2r_col(c2r_slot(threadIdx.x)), sub = c2r_sub(threadIdx.x);
     const float2 wc = conjf2(__ldg(tw.w32768 + col));  // W_32768^-col
-    __syncthreads();                                    // tables loaded
-    const LastTw lt = last_tw(T);                       // once per CTA
+    tc5::fence_before();
+    __syncthreads();  // tables loaded, barriers and tensor memory ready
+    tc5::fence_after();
+    const uint32_t quarter = P.tmem + (static_cast<uint32_t>(warp & 3) << 21);
+    const uint32_t park = quarter + kColPark + 64u * (warp >> 2), tw2nd = quarter + kColTw2;
+    if (warp < 4) {
+        float2 w[32];
+        pass2_twiddles(T, w);
+        tc5::tmem_park<32>(tw2nd, w);
+    }
+    tc5::fence_before();
+    __syncthreads();  // the four warps of a quarter read one table
+    tc5::fence_after();
+    const LastTw lt = last_tw(T);  // once per CTA
     const int64_t n_items = S.n_items;
-    auto src_of = [&](int64_t item) {
+    const int64_t G = gridDim.x;
+    auto fetch = [&](int64_t item, int buf) {  // one thread
         const SegA &g = S.s[seg_of(S, item)];
         const int64_t local = item - g.item0;
         const int64_t pol = local >= g.n_snaps, s = local - pol * g.n_snaps;  // n_pols <= 2: no division
-        return reinterpret_cast<const uint4 *>(g.spec + pol * g.spec_pol_stride + (g.snap0 + s) * kGroups);
+        tc5::bulk_g2s(sp + buf * kGroups, g.spec + pol * g.spec_pol_stride + (g.snap0 + s) * kGroups,
+                      kGroups * sizeof(uint32_t), &P.full[buf]);
+    };
+    auto wait = [&](uint64_t *bar, uint32_t parity) { tc5::wait_or_flag(bar, parity, &P.err); };
+    // Input columns of the k-th item (its spectrum in buffer k & 1), DFT-32,
+    // parked.  The first pass takes Z[col + 512 r] from the packed bins X[k]
+    // (k < 16384; the Nyquist bin X[16384] = 0, Im X[0] dropped), each
+    // Hermitian pair once with its mirror half from lane ^ 16.
+    auto input = [&](uint32_t k) {
+        wait(&P.full[k & 1], k >> 1);
+        const uint32_t *cur = sp + (k & 1) * kGroups;
+        float2 v[32], w[16];
+        for_r(std::make_integer_sequence<int, 16>{}, [&](auto pc) { w[decltype(pc)::value] = c2r_tw<decltype(pc)::value>(wc); });
+        c2r_paired<true>(
+            v, col, w, c2r_tw<16>(wc), [&](auto pc) { return nib_value(cur, col + kNTA * decltype(pc)::value); },
+            [&](auto pc) {
+                constexpr int p = decltype(pc)::value;
+                const int j = kMA - col - kNTA * p;  // 16384 only for col = 0, p = 0 (replaced by 0)
+                return nib_value(cur, p == 0 ? (j & (kMA - 1)) : j);
+            });
+        dft<32, true>(v);
+        tc5::tmem_park<32>(park, v);
     };
     int64_t item = blockIdx.x;
-    if (item < n_items) cp_async16(sp + 4 * threadIdx.x, src_of(item) + threadIdx.x);
-    cp_async_commit();
-    for (int buf = 0; item < n_items; item += gridDim.x, buf ^= 1) {
-        const int64_t next = item + gridDim.x;
-        if (next < n_items) cp_async16(sp + (buf ^ 1) * kGroups + 4 * threadIdx.x, src_of(next) + threadIdx.x);
-        cp_async_commit();
-        cp_async_wait_1();
-        __syncthreads();  // this item's spectrum landed; tables loaded
-        const uint32_t *cur = sp + buf * kGroups;
+    if (threadIdx.x == 0) {
+        if (item < n_items) fetch(item, 0);
+        if (item + G < n_items) fetch(item + G, 1);
+    }
+    if (item < n_items) input(0);
+    float2 *first = sm, *second = sm + kBlkA, *spare = sm + 2 * kBlkA;
+    for (uint32_t k = 0; item < n_items; item += G, ++k) {
+        float2 *mine = warp < 8 ? first : second;
+        {
+            float2 v[32];
+            tc5::tmem_unpark<32>(park, v);
+            if (warp >= 8 && k > 0) wait(&P.read, k - 1);
+            inv_store1(mine + kSub * blk_index(col & 15), col, v);
+        }
+        bar_sync(1 + (threadIdx.x >> 6), 64);
+        inv_pass2(mine + kSub * blk_index(sub), [&](float2 *v) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                float2 w[16];
+                tc5::tmem_unpark<16>(tw2nd + 32 * h, w);
+#pragma unroll
+                for (int r = 0; r < 16; ++r)
+                    if (16 * h + r > 0) v[16 * h + r] = cmulc(v[16 * h + r], w[r]);
+            }
+        });
+        __syncwarp();
+        if (lane == 0) tc5::mbar_arrive(&P.second);
+        if (item + G < n_items) input(k + 1);
+        wait(&P.second, k);
+        // every warp is done with this item's spectrum (its input columns
+        // came before its second pass): the buffer takes the item after next
+        if (threadIdx.x == 0 && item + 2 * G < n_items) fetch(item + 2 * G, k & 1);
         const SegA &g = S.s[seg_of(S, item)];
         const int64_t local = item - g.item0;
         const int64_t pol = local >= g.n_snaps, s = local - pol * g.n_snaps;
         float2 *dst = reinterpret_cast<float2 *>(g.out + pol * g.out_pol_stride + s * kNA);
-        // The inverse's first pass forms Z[col + 512 r] from the packed bins
-        // X[k] (k < 16384; the Nyquist bin X[16384] = 0, Im X[0] dropped), each
-        // Hermitian pair once with its mirror half from lane ^ 16: no pairing
-        // pass, no barrier of its own.
-        auto zin = [&](float2 *v) {
-            c2r_paired<true>(
-                v, col, wc, [&](auto pc) { return nib_value(cur, col + kNTA * decltype(pc)::value); },
-                [&](auto pc) {
-                    constexpr int p = decltype(pc)::value;
-                    const int k = kMA - col - kNTA * p;  // 16384 only for col = 0, p = 0 (replaced by 0)
-                    return nib_value(cur, p == 0 ? (k & (kMA - 1)) : k);
-                });
-        };
-        auto epi = [&](int jj, const float2 *u) {
+        inv_pass3(
+            [&](int r) { return (blk_second(r) ? second : first) + kSub * blk_index(r); }, lt,
+            [&](int jj, const float2 *u) {
 #pragma unroll
-            for (int r = 0; r < 16; ++r) __stcs(dst + jj + 1024 * r, u[r]);
-        };
-        // zin reads the packed spectrum (`cur`), not `sm`, and the barrier at
-        // the top of this loop follows the previous item's last reads of `sm`
-        ifft16384<false>(sm, T, zin, epi, col, lt);
+                for (int r = 0; r < 16; ++r) __stcs(dst + jj + 1024 * r, u[r]);
+            },
+            [&] {
+                __syncwarp();
+                if (lane == 0) tc5::mbar_arrive(&P.read);
+            });
+        float2 *t = first;
+        first = spare;
+        spare = second;
+        second = t;
     }
+    tc5::fence_before();
+    __syncthreads();
+    if (warp == 0) tc5::tmem_free(P.tmem, kColsA);
+    if (threadIdx.x == 0 && tc5::flag_set(&P.err)) *reinterpret_cast<volatile int *>(tw.status) = 1;
 }
 
 // ---------------------------------------------------------------------------
@@ -561,64 +701,250 @@ __global__ void __launch_bounds__(kNTA, 1) k_swarm_c2r(const __grid_constant__ S
 //   MODE 3: MODE 0, plus the (n, sum, sum of squares) of each chunk's
 //           floats (FP32 per thread and warp, FP64 across warps) to partials
 //           when the segment has them (windowed thresholds).
+//
+// The CTA's pipeline.  Each pass needs every warp's work of the pass before,
+// and the transform's buffer is rewritten while the next chunk waits for it;
+// every one of these dependencies is an mbarrier with one arrival per warp,
+// and the next chunk's first pass (radix 16), whose inputs come from global
+// memory and whose outputs wait in tensor memory, is done in three rounds
+// between the arrivals at and the waits for three of them.  Four teams of
+// four warps each take every fourth of eleven groups of 1664 elements through
+// passes 1 and 2: group m holds the first-pass butterflies j = 8 (m + 11 t) +
+// c (t < 13, c < 8) and the radix-13 blocks m + 11 c, so the two passes need
+// a team's barrier only.  A round's inputs (16 rows of 13 x 8 complex values
+// per team) are copied to shared memory by cp.async one round ahead: no
+// registers and, bypassing L1, none of its lines are held by loads in flight
+// (reading them with plain loads cost 9% of the kernel once L1 is small, as
+// beside stage A's shared memory).
+struct PipeB {
+    uint64_t xfree;   // the inverse's last-pass loads are done
+    uint64_t pass2, pass3, pass4;  // forward passes stored
+    uint64_t taken;   // the inverse has read X
+    uint64_t inv2;    // the inverse's second pass is stored
+    uint32_t tmem;
+    int err;
+};
+// Tensor memory columns: three parked rounds (32 columns for each of the four
+// warps of a lane quarter), the inverse's second-pass twiddles (the same for
+// the four), its last pass's bases (12 values, for each).
+constexpr uint32_t kColRound = 0, kColTw2B = 384, kColLast = 448, kColsB = 512;
+// One staged round of a team: row r (16) holds inputs t < 8 then, eight slots
+// further on, t >= 8, so that a half-warp (t and t + 8, c = 0..7) reads 16
+// bank pairs.
+constexpr int kStageRow = 13 * 8 + 8;
+constexpr int kStage = 16 * kStageRow;
+constexpr size_t kSmemPipeB = kSmemB + 4 * kStage * sizeof(float2);
+static_assert(kSmemPipeB <= 232448 - 1024, "stage BC shared memory above 227 KB");
+
 template <int MODE>
 __global__ void __launch_bounds__(kNTB, 1) k_resample(const __grid_constant__ SegsB S, Twiddles tw) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    float2 *sm = reinterpret_cast<float2 *>(smem_raw);
+    float2 *stages = reinterpret_cast<float2 *>(smem_raw);  // 16-byte aligned rows
+    float2 *sm = stages + 4 * kStage;
     float2 *tb = sm + kPadB;
     TabsA TA = tabs_a_at(tb);
     TabsB TB = tabs_b_at(tb, tw);
     __shared__ double red[64];
+    __shared__ PipeB P;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid == 0) {
+        uint64_t *bars[6] = {&P.xfree, &P.pass2, &P.pass3, &P.pass4, &P.taken, &P.inv2};
+        for (uint64_t *b : bars) tc5::mbar_init(b, kNTB / 32);
+        tc5::fence_mbar_init();
+        P.err = 0;
+    }
+    if (warp == 0) tc5::tmem_alloc(&P.tmem, kColsB);
     load_tabs_a(TA, tw);
     load_tabs_b(TB, tw);
-    const int tid = threadIdx.x;
-    const float2 wc = conjf2(__ldg(tw.w32768 + tid));  // W_32768^-tid
-    const int64_t n_items = S.n_items;
-    for (int64_t item = blockIdx.x; item < n_items; item += gridDim.x) {
+    // the inverse's first-pass column: warp w takes those of sub-transform w,
+    // so its first two passes need no barrier but the warp's own
+    const int sub = warp, col = sub + 16 * lane;
+    const float2 wc = conjf2(__ldg(tw.w32768 + col));  // W_32768^-col
+    tc5::fence_before();
+    __syncthreads();  // tables loaded, barriers and tensor memory ready
+    tc5::fence_after();
+    const uint32_t quarter = P.tmem + (static_cast<uint32_t>(warp & 3) << 21);
+    const uint32_t tw2nd = quarter + kColTw2B, twlast = quarter + kColLast + 16u * (warp >> 2);
+    {
+        float2 w[32];
+        if (warp < 4) {
+            pass2_twiddles(TA, w);
+            tc5::tmem_park<32>(tw2nd, w);
+        }
+        const LastTw lt = last_tw(TA);
+        float2 l[8];
+        l[0] = l[7] = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int j = 1; j < 4; ++j) {
+            l[j] = lt.S0[j];
+            l[3 + j] = lt.A0[j];
+        }
+        tc5::tmem_park<8>(twlast, l);
+    }
+    tc5::fence_before();
+    __syncthreads();  // the four warps of a quarter read one table
+    tc5::fence_after();
+    const int64_t n_items = S.n_items, G = gridDim.x;
+    auto wait = [&](uint64_t *bar, uint32_t parity) { tc5::wait_or_flag(bar, parity, &P.err); };
+    auto arrive = [&](uint64_t *bar) {
+        __syncwarp();
+        if (lane == 0) tc5::mbar_arrive(bar);
+    };
+    auto src_of = [&](int64_t item) {
+        const SegB &g = S.s[seg_of(S, item)];
+        const int64_t local = item - g.item0;
+        const int64_t pol = local >= g.n_chunks;  // n_pols <= 2: no division
+        return reinterpret_cast<const float2 *>(g.in + pol * g.in_pol_stride + (local - pol * g.n_chunks) * kNB);
+    };
+    // first two forward passes: this thread's team, its butterfly (c, t) of a
+    // group in pass 1 and its radix-13 column (block m + 11 c13, k13) in pass 2
+    const int team = warp >> 2, tt = tid & 127;
+    const int c1 = tt & 7, t1 = (tt >> 4) + (tt & 8), c13 = tt >> 4, k13 = tt & 15;
+    float2 *stg = stages + team * kStage;
+    auto team_sync = [&] { bar_sync(1 + team, 128); };
+    // Groups of this team, round by round.  Team 0 has one fewer: its warps
+    // have one more unit of the last forward pass than the others.
+    const int m0 = (team + 3) & 3;
+    // The inputs of round r (group m0 + 4 r) to the team's stage: 16 rows of
+    // 13 runs of 64 bytes, eight threads a row.
+    const int frow = tt >> 3, fpart = 2 * (tt & 3), ft = (tt >> 2) & 1;
+    float2 *fdst = stg + frow * kStageRow + 8 * ft + fpart;
+    const int fsrc = 1144 * frow + 8 * (m0 + 11 * ft) + fpart;
+    auto fetch = [&](const float2 *z, int r) {
+        if (m0 + 4 * r < 11) {
+            const float2 *src = z + fsrc + 32 * r;
+#pragma unroll
+            for (int j = 0; j < 7; ++j)  // runs t = ft + 2 j < 13
+                if (j < 6 || ft == 0) tc5::cp_async16(fdst + 16 * j + (j < 4 ? 0 : 8), src + 176 * j);
+        }
+        tc5::cp_async_commit();
+    };
+    // Round r of the first pass from the stage, parked; then the next fetch.
+    auto first_pass = [&](int r, const float2 *znext, int rnext) {
+        tc5::cp_async_wait_all();
+        team_sync();  // the whole team's copies landed
+        if (m0 + 4 * r < 11) {
+            float2 v[16];
+            const float2 *p = stg + (t1 < 13 ? 8 * t1 + (t1 < 8 ? 0 : 8) : 0) + c1;
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] = p[kStageRow * i];
+            dft<16, false>(v);
+            tc5::tmem_park<16>(quarter + kColRound + 96u * (warp >> 2) + 32u * r, v);
+        }
+        team_sync();  // the stage has been read
+        if (znext) fetch(znext, rnext);
+    };
+    int64_t item = blockIdx.x;
+    if (item < n_items) {
+        const float2 *z = src_of(item), *zn = item + G < n_items ? src_of(item + G) : nullptr;
+        fetch(z, 0);
+        first_pass(0, z, 1);
+        first_pass(1, z, 2);
+        first_pass(2, zn, 0);
+    }
+    for (uint32_t k = 0; item < n_items; item += G, ++k) {
         const SegB &g = S.s[seg_of(S, item)];
         const ResampleOut &o = g.o;
         const int n_chunks = g.n_chunks, skip = g.skip;
         const int64_t local = item - g.item0;
         const int pol = local >= n_chunks;  // n_pols <= 2: no division
         const int64_t c = local - pol * n_chunks;
-        __syncthreads();  // tables loaded / previous item's last smem reads done
-        const float2 *z = reinterpret_cast<const float2 *>(g.in + pol * g.in_pol_stride + c * kNB);
-        // forward 18304 with the R2C pairing in its last pass: X[q], q <= 18304
-        fft18304_from_global<true>(sm, z, TB);
-        // The next item's 146 KB chunk to L2 while this chunk's inverse runs,
-        // as nine bulk prefetches from nine threads: pass 1 of the next
-        // forward then reads from L2, not HBM.  Per-thread prefetch
-        // instructions (9 per thread) cost about 1k cycles of issue per chunk
-        // and gained 0.5%; prefetching at the start of the chunk, or two
-        // chunks ahead, gained less.
-        if (item + gridDim.x < n_items) {
-            const int64_t nx = item + gridDim.x;
-            const SegB &gn = S.s[seg_of(S, nx)];
-            const int64_t ln = nx - gn.item0;
-            const int64_t pn = ln >= gn.n_chunks;
-            const char *zn = reinterpret_cast<const char *>(gn.in + pn * gn.in_pol_stride + (ln - pn * gn.n_chunks) * kNB);
-            if (tid < 9) {  // 146432 B = 8 x 16384 + 15360, 16-byte aligned pieces
-                const uint32_t bytes = tid < 8 ? 16384u : static_cast<uint32_t>(kNB * 4 - 8 * 16384);
-                asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(zn + 16384 * tid), "r"(bytes) : "memory");
+        const bool more = item + G < n_items;
+        const float2 *zn = more ? src_of(item + G) : nullptr;
+        // forward 18304: the parked first pass into X, then radix 13
+        if (k > 0) wait(&P.xfree, k - 1);
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+            const int m = m0 + 4 * r;
+            if (m < 11) {
+                float2 v[16];
+                tc5::tmem_unpark<16>(quarter + kColRound + 96u * (warp >> 2) + 32u * r, v);
+                // rho(8g + c) = g/11 + 13 (g%11) + 143 c; padb(16 rho + r) = 17 rho + r (r < 16)
+                float2 *d = sm + 17 * (t1 + 13 * m + 143 * c1);
+                if (t1 < 13) {
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) d[i] = v[i];
+                }
             }
         }
-        // The inverse's first pass loads Z'[j], j = tid + 512 r, computed on the
+        team_sync();
+        {
+            float2 w13[13];
+            pass13_twiddles(TB, k13, w13);
+            for (int m = m0; m < 11; m += 4) fwd_pass13(sm, w13, m + 11 * c13, k13);
+        }
+        arrive(&P.pass2);
+        if (more) first_pass(0, zn, 1);
+        wait(&P.pass2, k);
+        fwd_pass11(sm, TB);
+        arrive(&P.pass3);
+        if (more) first_pass(1, zn, 2);
+        wait(&P.pass3, k);
+        // the last forward pass with the R2C pairing: X[q], q <= 18304
+        fwd_pass8<true>(sm, TB);
+        arrive(&P.pass4);
+        wait(&P.pass4, k);
+        // The chunk after next, 146 KB, to L2 as nine bulk prefetches from nine threads
+        if (item + 2 * G < n_items && tid < 9) {  // 146432 B = 8 x 16384 + 15360, 16-byte aligned pieces
+            const uint32_t bytes = tid < 8 ? 16384u : static_cast<uint32_t>(kNB * 4 - 8 * 16384);
+            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(
+                             reinterpret_cast<const char *>(src_of(item + 2 * G)) + 16384 * tid),
+                         "r"(bytes)
+                         : "memory");
+        }
+        // The inverse's first pass loads Z'[j], j = col + 512 r, computed on the
         // fly by the C2R pairing of the window Y[j] = X[skip + j], j = 0..16384
-        // (no pass of its own; ifft16384 syncs before its first stores), with
-        // W_32768^-j = wc e^{2 pi i r/64} (wc per thread, the rest compile-time);
-        // Im Y[0] and Im Y[16384] are dropped.
+        // (no pass of its own), with W_32768^-j = wc e^{2 pi i r/64} (wc per
+        // thread, the rest compile-time); Im Y[0] and Im Y[16384] are dropped.
+        // A warp's columns are 16 apart, one padded row of `sm` each: both
+        // runs, up from Y[col] and down from Y[16384 - col], are conflict-free.
         auto zin = [&](float2 *v) {
-            const float2 *lo = sm + padb(skip + tid);        // Y[tid + 512 r] = lo[544 r]
-            const float2 *hi = sm + padb(skip + kMA - tid);  // Y[16384 - tid - 512 r] = hi[-544 r]
+            const float2 *lo = sm + padb(skip + col);        // Y[col + 512 r] = lo[544 r]
+            const float2 *hi = sm + padb(skip + kMA - col);  // Y[16384 - col - 512 r] = hi[-544 r]
             for_r(std::make_integer_sequence<int, 32>{}, [&](auto rc) {
                 constexpr int r = decltype(rc)::value;
-                v[r] = c2r_pre(lo[544 * r], hi[-544 * r], tid + 512 * r, c2r_tw<r>(wc));
+                v[r] = c2r_pre<0, r == 0 ? 1 : 0>(lo[544 * r], hi[-544 * r], col + 512 * r, c2r_tw_rn<r>(wc));
             });
+        };
+        auto inverse = [&](auto epi) {
+            {
+                float2 v[32];
+                zin(v);
+                arrive(&P.taken);
+                dft<32, true>(v);
+                wait(&P.taken, k);  // every read of X ends before the first stores over it
+                inv_store1(sm + kSub * sub, col, v);
+            }
+            __syncwarp();
+            inv_pass2(sm + kSub * sub, [&](float2 *v) {
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    float2 w[16];
+                    tc5::tmem_unpark<16>(tw2nd + 32 * h, w);
+#pragma unroll
+                    for (int r = 0; r < 16; ++r)
+                        if (16 * h + r > 0) v[16 * h + r] = cmulc(v[16 * h + r], w[r]);
+                }
+            });
+            arrive(&P.inv2);
+            if (more) first_pass(2, item + 2 * G < n_items ? src_of(item + 2 * G) : nullptr, 0);
+            LastTw lt;
+            {
+                float2 l[8];
+                tc5::tmem_unpark<8>(twlast, l);
+#pragma unroll
+                for (int j = 1; j < 4; ++j) {
+                    lt.S0[j] = l[j];
+                    lt.A0[j] = l[3 + j];
+                }
+            }
+            wait(&P.inv2, k);
+            inv_pass3([&](int r) { return sm + kSub * r; }, lt, epi, [&] { arrive(&P.xfree); });
         };
         if constexpr (MODE == 0 || MODE == 3) {
             uint32_t *words = reinterpret_cast<uint32_t *>(o.out + pol * o.out_pol_stride +
                                                            (o.pkt0 + c) * o.pkt_stride + o.payload_off);
-            const float th = o.thr[pol], off = o.thr[2 + pol];
+            const Coder2 cd = coder2(o.thr[pol], o.thr[2 + pol]);
             float f1 = 0.f, f2 = 0.f;
             // Word (jj >> 3) + 128 r holds the 4-bit codes of outputs jj + 1024 r
             // of the 8 lanes jj & 7 = c (lane c at bits 4c).  Each lane builds
@@ -628,10 +954,14 @@ __global__ void __launch_bounds__(kNTB, 1) k_resample(const __grid_constant__ Se
             auto epi = [&](int jj, const float2 *u) {
                 uint32_t wl = 0, wh = 0;
 #pragma unroll
-                for (int r = 0; r < 8; ++r) {
-                    wl |= (code2(u[r].x, th, off) | (code2(u[r].y, th, off) << 2)) << (4 * r);
-                    wh |= (code2(u[8 + r].x, th, off) | (code2(u[8 + r].y, th, off) << 2)) << (4 * r);
+                for (int r = 7; r >= 0; --r) {
+                    push2(wl, u[r].y, cd);
+                    push2(wl, u[r].x, cd);
+                    push2(wh, u[8 + r].y, cd);
+                    push2(wh, u[8 + r].x, cd);
                 }
+                wl = codes2(wl);
+                wh = codes2(wh);
                 if constexpr (MODE == 3) {
 #pragma unroll
                     for (int r = 0; r < 16; ++r) {
@@ -645,7 +975,7 @@ __global__ void __launch_bounds__(kNTB, 1) k_resample(const __grid_constant__ Se
                 words[(jj >> 3) + 128 * c] = wl;
                 words[(jj >> 3) + 128 * (8 + c)] = wh;
             };
-            ifft16384(sm, TA, zin, epi);
+            inverse(epi);
             if constexpr (MODE == 3) {
                 if (o.partials != nullptr) {  // uniform over the block
                     double s1, s2;
@@ -672,7 +1002,7 @@ __global__ void __launch_bounds__(kNTB, 1) k_resample(const __grid_constant__ Se
                     }
                 }
             };
-            ifft16384(sm, TA, zin, epi);
+            inverse(epi);
             if constexpr (MODE == 1) {
                 block_sum2(s1, s2, red);
                 if (tid == 0) {
@@ -686,6 +1016,10 @@ __global__ void __launch_bounds__(kNTB, 1) k_resample(const __grid_constant__ Se
             }
         }
     }
+    tc5::fence_before();
+    __syncthreads();
+    if (warp == 0) tc5::tmem_free(P.tmem, kColsB);
+    if (tid == 0 && tc5::flag_set(&P.err)) *reinterpret_cast<volatile int *>(tw.status) = 1;
 }
 
 // SwarmR2C alone: complex64 [n][18305] spectra (persistent over chunks).
@@ -698,7 +1032,7 @@ __global__ void __launch_bounds__(kNTB, 1)
     load_tabs_b(TB, tw);
     for (int64_t c = blockIdx.x; c < n_chunks; c += gridDim.x) {
         __syncthreads();
-        fft18304_from_global<false>(sm, reinterpret_cast<const float2 *>(in + c * kNB), TB);
+        fft18304_from_global(sm, reinterpret_cast<const float2 *>(in + c * kNB), TB);
         float2 *dst = out + c * (kMB + 1);
         for (int q = threadIdx.x; q <= kMB; q += kNTB) dst[q] = r2c_bin(sm, q, __ldg(tw.w36608 + q));
     }
@@ -716,7 +1050,6 @@ __global__ void __launch_bounds__(kNTB, 1)
     const int tid = threadIdx.x;
     const float2 wc = conjf2(__ldg(tw.w32768 + tid));
     for (int64_t c = blockIdx.x; c < n_chunks; c += gridDim.x) {
-        __syncthreads();
         const float2 *y = in + c * in_stride + skip;
         auto zin = [&](float2 *v) {
             for_r(std::make_integer_sequence<int, 32>{}, [&](auto rc) {
@@ -730,7 +1063,22 @@ __global__ void __launch_bounds__(kNTB, 1)
 #pragma unroll
             for (int r = 0; r < 16; ++r) dst[jj + 1024 * r] = u[r];
         };
-        ifft16384(sm, TA, zin, epi);
+        float2 v[32];
+        zin(v);
+        dft<32, true>(v);
+        __syncthreads();  // the previous chunk's last reads of `sm` (and the table loads) are done
+        // consecutive columns (coalesced reads): a sub-transform's first two
+        // passes span all warps
+        inv_store1(sm + kSub * (tid & 15), tid, v);
+        __syncthreads();
+        inv_pass2(sm + kSub * (tid >> 5), [&](float2 *v) {
+            float2 w[32];
+            pass2_twiddles(TA, w);
+#pragma unroll
+            for (int r = 1; r < 32; ++r) v[r] = cmulc(v[r], w[r]);
+        });
+        __syncthreads();
+        inv_pass3([&](int r) { return sm + kSub * r; }, last_tw(TA), epi, [] {});
     }
 }
 
@@ -968,13 +1316,13 @@ cudaError_t configure_fft_kernels() {
     cudaError_t e;
     if ((e = cudaFuncSetAttribute(k_swarm_c2r, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemA))) != cudaSuccess)
         return e;
-    if ((e = cudaFuncSetAttribute(k_resample<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemB))) != cudaSuccess)
+    if ((e = cudaFuncSetAttribute(k_resample<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemPipeB))) != cudaSuccess)
         return e;
-    if ((e = cudaFuncSetAttribute(k_resample<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemB))) != cudaSuccess)
+    if ((e = cudaFuncSetAttribute(k_resample<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemPipeB))) != cudaSuccess)
         return e;
-    if ((e = cudaFuncSetAttribute(k_resample<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemB))) != cudaSuccess)
+    if ((e = cudaFuncSetAttribute(k_resample<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemPipeB))) != cudaSuccess)
         return e;
-    if ((e = cudaFuncSetAttribute(k_resample<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemB))) != cudaSuccess)
+    if ((e = cudaFuncSetAttribute(k_resample<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemPipeB))) != cudaSuccess)
         return e;
     if ((e = cudaFuncSetAttribute(k_swarm_r2c, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemB))) != cudaSuccess)
         return e;
@@ -1007,13 +1355,13 @@ cudaError_t launch_resample_segs(int mode, const SegsB &S, const Twiddles &tw, c
     if (S.n < 1 || S.n > kMaxSegs) return cudaErrorInvalidValue;
     const unsigned grid = persistent_grid(S.n_items);
     if (mode == 0)
-        k_resample<0><<<grid, kNTB, kSmemB, st>>>(S, tw);
+        k_resample<0><<<grid, kNTB, kSmemPipeB, st>>>(S, tw);
     else if (mode == 3)
-        k_resample<3><<<grid, kNTB, kSmemB, st>>>(S, tw);
+        k_resample<3><<<grid, kNTB, kSmemPipeB, st>>>(S, tw);
     else if (mode == 1)
-        k_resample<1><<<grid, kNTB, kSmemB, st>>>(S, tw);
+        k_resample<1><<<grid, kNTB, kSmemPipeB, st>>>(S, tw);
     else
-        k_resample<2><<<grid, kNTB, kSmemB, st>>>(S, tw);
+        k_resample<2><<<grid, kNTB, kSmemPipeB, st>>>(S, tw);
     return cudaGetLastError();
 }
 

@@ -730,15 +730,12 @@ int tc_prepare(sdbe_resampler *h, cudaStream_t st) {
     if (cudaMalloc(&h->tc_f128, f128.size() * sizeof(__half)) != cudaSuccess ||
         cudaMalloc(&h->tc_f143, f143.size() * sizeof(__half)) != cudaSuccess ||
         cudaMalloc(&h->tc_bufx, 2 * wave_snaps * kMA * sizeof(float2)) != cudaSuccess ||
-        cudaMalloc(&h->tc_bufy, 2 * wave_chunks * kMB * sizeof(float2)) != cudaSuccess ||
-        cudaHostAlloc(&h->tc_status_host, sizeof(int), cudaHostAllocMapped) != cudaSuccess) {
+        cudaMalloc(&h->tc_bufy, 2 * wave_chunks * kMB * sizeof(float2)) != cudaSuccess) {
         cudaGetLastError();
         return fail(h, SDBE_ERR_NOMEM, "cannot allocate the tensor-core scratch");
     }
     SDBE_CK(h, cudaMemcpyAsync(h->tc_f128, f128.data(), f128.size() * sizeof(__half), cudaMemcpyHostToDevice, st));
     SDBE_CK(h, cudaMemcpyAsync(h->tc_f143, f143.data(), f143.size() * sizeof(__half), cudaMemcpyHostToDevice, st));
-    *h->tc_status_host = 0;
-    SDBE_CK(h, cudaHostGetDevicePointer(reinterpret_cast<void **>(&h->tc_status), h->tc_status_host, 0));
     SDBE_CK(h, cudaStreamSynchronize(st));  // the host tables are freed on return
     return SDBE_OK;
 }
@@ -756,8 +753,7 @@ int tc_wave_multi(const std::vector<TcWaveItem> &w, bool first, cudaStream_t st)
     if (tc_splits(h0) == 2) return tcf_wave_multi(w, first, st);  // SDBE_PRECISION_TC16_FAST (k_tcf.cu)
     for (const auto &it : w) {
         if (int rc = tc_prepare(it.h, st)) return rc;
-        if (*reinterpret_cast<volatile int *>(it.h->tc_status_host))  // written by an earlier call's kernels
-            return fail(it.h, SDBE_ERR_CUDA, "a tensor-core transform timed out on its mbarrier wait");
+        if (int rc = check_status(it.h)) return rc;
     }
     const Twiddles &tw = h0->tw;
     const uint8_t *f128 = static_cast<const uint8_t *>(h0->tc_f128);

@@ -131,16 +131,6 @@ __device__ __forceinline__ float2 acc2(const uint32_t *r, int i) {
     return make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
 }
 
-// Bulk copy global -> shared of `bytes` (multiple of 16), completing on mbar.
-__device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t bytes, uint64_t *mbar) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(mbar)), "r"(bytes)
-                 : "memory");
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
-        "l"(src), "r"(bytes), "r"(smem_u32(mbar))
-        : "memory");
-}
-
 // Bulk copy shared -> global of `bytes` (multiple of 16) in this thread's
 // bulk group; the source may be rewritten after bulk_wait_read().
 __device__ __forceinline__ void bulk_s2g(void *dst, const void *src, uint32_t bytes) {
@@ -326,15 +316,6 @@ __device__ __forceinline__ void bump(unsigned *p) {
 }
 // Generic-proxy accesses ordered with this thread's bulk (async-proxy) copies of global memory.
 __device__ __forceinline__ void fence_proxy_global() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
-
-__device__ __forceinline__ void tmem_alloc_cols(uint32_t *dst) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst)),
-                 "r"(kTmemCols));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-}
-__device__ __forceinline__ void tmem_free_cols(uint32_t base) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(kTmemCols));
-}
 
 // Shared item slots of a chain phase: [t] team t's current item, its issuer's
 // mark (< 0: end), [2 + 4 t + 2 p ..] team t's (item, next) pair p, [10 + s %
@@ -1045,13 +1026,13 @@ __global__ void __launch_bounds__(kInvThreads, 1) k_tcf_inv(const __grid_constan
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *sm = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     const int warp = threadIdx.x >> 5;
-    if (warp == 0) tmem_alloc_cols(&g_tmem_base);
+    if (warp == 0) tmem_alloc(&g_tmem_base, kTmemCols);
     fence_before();
     __syncthreads();
     fence_after();
     const uint32_t tb = g_tmem_base;
     inv_phase<IN, OUT, 0, false>(a, Sched{nullptr, nullptr, nullptr}, sm, tb);
-    if (warp == 0) tmem_free_cols(tb);
+    if (warp == 0) tmem_free(tb, kTmemCols);
 }
 
 // ============================================================================
@@ -1462,13 +1443,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_tcf_fwd(const __grid_constant__
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *sm = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     const int warp = threadIdx.x >> 5;
-    if (warp == 0) tmem_alloc_cols(&g_tmem_base);
+    if (warp == 0) tmem_alloc(&g_tmem_base, kTmemCols);
     fence_before();
     __syncthreads();
     fence_after();
     const uint32_t tb = g_tmem_base;
     fwd_phase<false>(a, Sched{nullptr, nullptr, nullptr}, sm, tb);
-    if (warp == 0) tmem_free_cols(tb);
+    if (warp == 0) tmem_free(tb, kTmemCols);
 }
 
 // Stages A, B and C of one wave in one persistent launch: every CTA runs the
@@ -1489,7 +1470,7 @@ __global__ void __launch_bounds__(kInvThreads, 1) k_tcf_chain(const __grid_const
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *sm = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     const int warp = threadIdx.x >> 5;
-    if (warp == 0) tmem_alloc_cols(&g_tmem_base);
+    if (warp == 0) tmem_alloc(&g_tmem_base, kTmemCols);
     fence_before();
     __syncthreads();
     fence_after();
@@ -1498,7 +1479,7 @@ __global__ void __launch_bounds__(kInvThreads, 1) k_tcf_chain(const __grid_const
     inv_phase<IN_PACKED, OUT_TS_HALF, 0, true>(c.A, Sched{c.q, nullptr, dep_a}, sm, tb);
     fwd_phase<true>(c.B, Sched{c.q + 1, dep_a, done_b}, sm, tb);
     inv_phase<IN_BINS, OUTC, 1, true>(c.C, Sched{c.q + 2, done_b, nullptr}, sm, tb);
-    if (warp == 0) tmem_free_cols(tb);
+    if (warp == 0) tmem_free(tb, kTmemCols);
 }
 
 // Float time series -> FP16 x 2^-2 (sdbe_resample_chunks in this form).
@@ -1645,17 +1626,9 @@ constexpr bool kFusedByDefault = true;        // stage_launches 0: one launch pe
 
 }  // namespace
 
-// Tables of the fast tensor-core kernels and the time-out flag, on first use.
+// Tables of the fast tensor-core kernels, on first use.
 int tcf_prepare(sdbe_resampler *h, cudaStream_t st) {
     if (h->tcf_tabs) return SDBE_OK;
-    if (!h->tc_status_host) {
-        if (cudaHostAlloc(&h->tc_status_host, sizeof(int), cudaHostAllocMapped) != cudaSuccess) {
-            cudaGetLastError();
-            return fail(h, SDBE_ERR_NOMEM, "cannot allocate the tensor-core status flag");
-        }
-        *h->tc_status_host = 0;
-        SDBE_CK(h, cudaHostGetDevicePointer(reinterpret_cast<void **>(&h->tc_status), h->tc_status_host, 0));
-    }
     const std::vector<uint8_t> blob = build_blob();
     if (blob.size() != kBlobBytes) return fail(h, SDBE_ERR_STATE, "tensor-core table layout mismatch");
     if (cudaMalloc(&h->tcf_tabs, blob.size()) != cudaSuccess) {
@@ -1780,8 +1753,7 @@ int tcf_wave_multi(const std::vector<TcWaveItem> &w, bool first, cudaStream_t st
     for (const auto &it : w) {
         sdbe_resampler *h = it.h;
         if (int rc = tcf_prepare(h, st)) return rc;
-        if (*reinterpret_cast<volatile int *>(h->tc_status_host))  // written by an earlier call's kernels
-            return fail(h, SDBE_ERR_CUDA, "a tensor-core transform timed out on its mbarrier wait");
+        if (int rc = check_status(h)) return rc;
         const int64_t per_pol = static_cast<int64_t>(h->wave) * kChunks;
         if (int rc = grow(h, reinterpret_cast<uint8_t **>(&h->tcf_bins), &h->tcf_bins_bytes,
                           2 * per_pol * kTcfBinsLen * 4, "the tensor-core bins"))

@@ -45,6 +45,19 @@ __host__ __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
 __host__ __device__ __forceinline__ float2 cmulc(float2 a, float2 b) {  // a * conj(b)
     return make_float2(a.x * b.x + a.y * b.y, a.y * b.x - a.x * b.y);
 }
+// a * b with the rounding pinned.  Of a component's two products one is
+// rounded and the other fused into the sum, or both are rounded; in cmul the
+// compiler chooses, and where the code around a product changes, its choice
+// (and the last bit of every later value) may change too.  X for the real
+// part: 0 rounds a.y b.y, 1 a.x b.x, 2 both; Y for the imaginary part: 0
+// rounds a.y b.x, 1 a.x b.y, 2 both.
+template <int X, int Y>
+__device__ __forceinline__ float2 cmul_rn(float2 a, float2 b) {
+    const float px = __fmul_rn(a.x, b.x), py = __fmul_rn(a.y, b.y), qx = __fmul_rn(a.x, b.y), qy = __fmul_rn(a.y, b.x);
+    return make_float2(
+        X == 0 ? __fmaf_rn(a.x, b.x, -py) : (X == 1 ? __fmaf_rn(-a.y, b.y, px) : __fsub_rn(px, py)),
+        Y == 0 ? __fmaf_rn(a.x, b.y, qy) : (Y == 1 ? __fmaf_rn(a.y, b.x, qx) : __fadd_rn(qx, qy)));
+}
 __host__ __device__ __forceinline__ float2 conjf2(float2 a) { return make_float2(a.x, -a.y); }
 
 // ---- twiddle tables (device, built once per handle) -----------------------
@@ -53,6 +66,7 @@ struct Twiddles {
     const float2 *w18304;  // exp(-2 pi i k / 18304), k < 18304
     const float2 *w32768;  // exp(-2 pi i k / 32768), k < 16384
     const float2 *w36608;  // exp(-2 pi i k / 36608), k <= 18304
+    int *status;           // set to 1 by a kernel whose barrier wait timed out (host-mapped)
 };
 
 // ---- error plumbing -------------------------------------------------------

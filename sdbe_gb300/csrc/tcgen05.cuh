@@ -124,6 +124,32 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *mbar, uint32_t parity, uint6
     }
 }
 
+__device__ __forceinline__ bool flag_set(const int *flag) { return *reinterpret_cast<const volatile int *>(flag) != 0; }
+// mbar_wait that raises `flag` (shared memory) on time-out; once it is raised, waits return at once.
+__device__ __forceinline__ void wait_or_flag(uint64_t *mbar, uint32_t parity, int *flag) {
+    if (mbar_poll(mbar, parity)) return;
+    if (flag_set(flag)) return;
+    if (!mbar_wait(mbar, parity)) *reinterpret_cast<volatile int *>(flag) = 1;
+}
+__device__ __forceinline__ void fence_mbar_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
+
+// 16 bytes global -> shared, not through L1.
+__device__ __forceinline__ void cp_async16(void *dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// Bulk copy global -> shared of `bytes` (multiple of 16), completing on mbar.
+__device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t bytes, uint64_t *mbar) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(mbar)), "r"(bytes)
+                 : "memory");
+    asm volatile(
+        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
+        "l"(src), "r"(bytes), "r"(smem_u32(mbar))
+        : "memory");
+}
+
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 // Generic-proxy shared-memory writes made visible to the tensor cores (async proxy).
@@ -171,6 +197,89 @@ __device__ __forceinline__ uint32_t sw128_off(int row, int kc) {
 __device__ __forceinline__ uint32_t sw64_off(int row, int kc) {
     return static_cast<uint32_t>((row >> 3) * 512 + (row & 7) * 64 + ((((kc >> 2) ^ ((row & 7) >> 1)) & 3) << 4) +
                                  (kc & 3) * 4);
+}
+
+// Tensor memory of `cols` columns (a power of two, 32 to 512), by one whole
+// warp; the base address lands in shared memory at dst.
+__device__ __forceinline__ void tmem_alloc(uint32_t *dst, uint32_t cols) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst)), "r"(cols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+}
+__device__ __forceinline__ void tmem_free(uint32_t base, uint32_t cols) {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(cols));
+}
+
+// 32 registers to or from 32 columns of this thread's lane (taddr as in tmem_ld16), no wait.
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const float *r) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15};" ::"f"(r[0]),
+        "f"(r[1]), "f"(r[2]), "f"(r[3]), "f"(r[4]), "f"(r[5]), "f"(r[6]), "f"(r[7]), "f"(r[8]), "f"(r[9]), "f"(r[10]),
+        "f"(r[11]), "f"(r[12]), "f"(r[13]), "f"(r[14]), "f"(r[15]), "r"(taddr)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_ldf16(uint32_t taddr, float *r) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]), "=f"(r[6]), "=f"(r[7]), "=f"(r[8]),
+          "=f"(r[9]), "=f"(r[10]), "=f"(r[11]), "=f"(r[12]), "=f"(r[13]), "=f"(r[14]), "=f"(r[15])
+        : "r"(taddr)
+        : "memory");
+}
+#define SDBE_RIN(r) \
+    "f"(r[0]), "f"(r[1]), "f"(r[2]), "f"(r[3]), "f"(r[4]), "f"(r[5]), "f"(r[6]), "f"(r[7]), \
+    "f"(r[8]), "f"(r[9]), "f"(r[10]), "f"(r[11]), "f"(r[12]), "f"(r[13]), "f"(r[14]), "f"(r[15]), \
+    "f"(r[16]), "f"(r[17]), "f"(r[18]), "f"(r[19]), "f"(r[20]), "f"(r[21]), "f"(r[22]), "f"(r[23]), \
+    "f"(r[24]), "f"(r[25]), "f"(r[26]), "f"(r[27]), "f"(r[28]), "f"(r[29]), "f"(r[30]), "f"(r[31])
+#define SDBE_ROUT(r) \
+    "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]), "=f"(r[6]), "=f"(r[7]), \
+    "=f"(r[8]), "=f"(r[9]), "=f"(r[10]), "=f"(r[11]), "=f"(r[12]), "=f"(r[13]), "=f"(r[14]), "=f"(r[15]), \
+    "=f"(r[16]), "=f"(r[17]), "=f"(r[18]), "=f"(r[19]), "=f"(r[20]), "=f"(r[21]), "=f"(r[22]), "=f"(r[23]), \
+    "=f"(r[24]), "=f"(r[25]), "=f"(r[26]), "=f"(r[27]), "=f"(r[28]), "=f"(r[29]), "=f"(r[30]), "=f"(r[31])
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const float *r) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%32], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,"
+        "%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31};" ::SDBE_RIN(r),
+        "r"(taddr)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float *r) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,"
+        "%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+        : SDBE_ROUT(r)
+        : "r"(taddr)
+        : "memory");
+}
+#undef SDBE_RIN
+#undef SDBE_ROUT
+// N complex values of this thread (N a multiple of 8) set aside in 2 N
+// columns of its lane, and taken back by the same thread.
+template <int N>
+__device__ __forceinline__ void tmem_park(uint32_t taddr, const float2 *v) {
+    float r[2 * N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        r[2 * i] = v[i].x;
+        r[2 * i + 1] = v[i].y;
+    }
+#pragma unroll
+    for (int i = 0; i + 16 <= N; i += 16) tmem_st32(taddr + 2 * i, r + 2 * i);
+    if constexpr (N % 16 == 8) tmem_st16(taddr + 2 * (N - 8), r + 2 * (N - 8));
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+template <int N>
+__device__ __forceinline__ void tmem_unpark(uint32_t taddr, float2 *v) {
+    float r[2 * N];
+#pragma unroll
+    for (int i = 0; i + 16 <= N; i += 16) tmem_ld32(taddr + 2 * i, r + 2 * i);
+    if constexpr (N % 16 == 8) tmem_ldf16(taddr + 2 * (N - 8), r + 2 * (N - 8));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        asm volatile("" : "+f"(r[2 * i]), "+f"(r[2 * i + 1]));  // no use moves above the wait
+        v[i] = make_float2(r[2 * i], r[2 * i + 1]);
+    }
 }
 
 // (a, b) -> the FP16 pair rn(a), rn(b) as a 32-bit word.
