@@ -62,7 +62,6 @@ void free_all(sdbe_resampler *h) {
     }
     cudaFree(h->tw_storage);
     cudaFree(h->spec);
-    cudaFree(h->bitmap);
     cudaFree(h->counts);
     cudaFree(h->ts);
     cudaFree(h->fout);
@@ -107,6 +106,10 @@ void free_all(sdbe_resampler *h) {
     if (h->copy_out) cudaStreamDestroy(h->copy_out);
     if (h->stream) cudaStreamDestroy(h->stream);
 }
+
+// Per-frame packet counts and the count of rejected packets, rounded up so
+// that the completion bitmap behind them is aligned (one fill clears both).
+size_t counts_bytes(int max_frames) { return ((static_cast<size_t>(max_frames) + 1) * sizeof(int32_t) + 255) / 256 * 256; }
 
 cudaStream_t pick(sdbe_resampler *h, void *stream) {
     return stream ? static_cast<cudaStream_t>(stream) : h->stream;
@@ -315,8 +318,8 @@ int prepare_call(CallPlan &c, UnpackSegs *batch = nullptr) {
         uint32_t *dst = mar ? h->raw : h->spec;
         const int64_t dst_stride = mar ? h->raw_pol_stride : h->spec_pol_stride;
         const int64_t snap0 = mar ? static_cast<int64_t>(h->raw_carry) * kSnapsPerFrame : h->carry;
-        SDBE_CK(h, cudaMemsetAsync(h->bitmap, 0, static_cast<size_t>(n_frames) * 256, st));
-        SDBE_CK(h, cudaMemsetAsync(h->counts, 0, (static_cast<size_t>(h->cfg.max_frames) + 1) * sizeof(int32_t), st));
+        // the counts and, behind them, the bitmap
+        SDBE_CK(h, cudaMemsetAsync(h->counts, 0, counts_bytes(h->cfg.max_frames) + static_cast<size_t>(n_frames) * 256, st));
         if (batch && !mar) {
             unpack_segs_add(*batch, UnpackSeg{static_cast<const uint8_t *>(src), c.n_packets, c.b_zero, n_frames, map,
                                               dst, dst_stride, snap0, h->bitmap, h->counts,
@@ -394,11 +397,9 @@ int complete_call(CallPlan &c, sdbe_result *result) {
     const int64_t total = h->carry + c.n_frames_out * kSnapsPerFrame;
     const int64_t new_carry = total - c.n_batches * kBatchSnaps;
     if (c.n_batches > 0 && new_carry > 0) {
-        for (int pol = 0; pol < 2; ++pol) {
-            uint32_t *base = h->spec + pol * h->spec_pol_stride;
-            SDBE_CK(h, cudaMemcpyAsync(base, base + c.n_batches * kBatchSnaps * kGroups,
-                                       new_carry * kGroups * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st));
-        }
+        const size_t pitch = static_cast<size_t>(h->spec_pol_stride) * sizeof(uint32_t);
+        SDBE_CK(h, cudaMemcpy2DAsync(h->spec, pitch, h->spec + c.n_batches * kBatchSnaps * kGroups, pitch,
+                                     new_carry * kGroups * sizeof(uint32_t), 2, cudaMemcpyDeviceToDevice, st));
     }
     h->carry = new_carry;
     h->last_stream = st;
@@ -508,7 +509,7 @@ int fft_chain_multi(std::vector<CallPlan> &cs) {
             for (int i : first) {
                 sdbe_resampler *h = cs[i].h;
                 const PayloadTarget &t = cs[i].pt;
-                SDBE_CK(h, launch_finalize_thresholds(h->partials, kChunks, h->cfg.pol1_uses_pol0_threshold, h->thr, st));
+                SDBE_CK(h, launch_finalize_thresholds(h->partials, h->cfg.pol1_uses_pol0_threshold, h->thr, st));
                 SDBE_CK(h, launch_quantize_chunks(h->fout, static_cast<int64_t>(kChunks) * kNC, kChunks, h->thr, t.base,
                                                   t.pol_stride, t.pkt_stride, t.payload_off, 0, st));
                 h->thresholds_set = true;
@@ -649,8 +650,8 @@ int sdbe_create(const sdbe_config *cfg, sdbe_resampler **out) {
         return bail(SDBE_ERR_CUDA, "status flag address");
     h->tw.status = h->tc_status;
     bool ok = cudaMalloc(&h->spec, 2 * h->spec_pol_stride * sizeof(uint32_t)) == cudaSuccess &&
-              cudaMalloc(&h->bitmap, static_cast<size_t>(cfg->max_frames) * 256) == cudaSuccess &&
-              cudaMalloc(&h->counts, (static_cast<size_t>(cfg->max_frames) + 1) * sizeof(int32_t)) == cudaSuccess &&
+              cudaMalloc(&h->counts, counts_bytes(cfg->max_frames) + static_cast<size_t>(cfg->max_frames) * 256) ==
+                  cudaSuccess &&
               cudaMalloc(&h->ts, 2 * h->ts_pol_stride * sizeof(float)) == cudaSuccess &&
               cudaMalloc(&h->fout, 2 * static_cast<size_t>(kChunks) * kNC * sizeof(float)) == cudaSuccess &&
               cudaMalloc(&h->partials, 2 * kChunks * 3 * sizeof(double)) == cudaSuccess &&
@@ -667,6 +668,7 @@ int sdbe_create(const sdbe_config *cfg, sdbe_resampler **out) {
         ok = cudaMalloc(&h->raw, 2 * h->raw_pol_stride * sizeof(uint32_t)) == cudaSuccess;
     }
     if (!ok) return bail(SDBE_ERR_NOMEM, "device buffer allocation failed");
+    h->bitmap = reinterpret_cast<uint32_t *>(reinterpret_cast<uint8_t *>(h->counts) + counts_bytes(cfg->max_frames));
     if (cudaMemset(h->thr, 0, 8 * sizeof(float)) != cudaSuccess) return bail(SDBE_ERR_CUDA, "memset");
     *out = h;
     return SDBE_OK;

@@ -343,16 +343,39 @@ __device__ __forceinline__ void block_sum2(double &a, double &b, double *scratch
         scratch[32 + warp] = b;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double sa = 0.0, sb = 0.0;
-        for (int w = 0; w < nw; ++w) {
-            sa += scratch[w];
-            sb += scratch[32 + w];
-        }
-        a = sa;
-        b = sb;
+    if (warp == 0) {
+        a = warp_sum(lane < nw ? scratch[lane] : 0.0);
+        b = warp_sum(lane < nw ? scratch[32 + lane] : 0.0);
     }
 }
+
+// One thread's sum and sum of squares of FP32 samples as unevaluated sums of
+// FP32 values (Knuth's two-sum; a square is its rounded value plus the exact
+// fma remainder), handed on in FP64: FP64 instructions, conversions included,
+// run at 1/64 of the FP32 rate, and seven of them for two samples took 28k of
+// a first-batch chunk's 65k cycles.  Two levels for the sum and three for the
+// squares leave the variance of a batch with the same error as FP64 sums
+// (1e-16 relative against exact sums; two levels for the squares: 5e-15).
+struct Moments2 {
+    float s = 0.f, se = 0.f, q = 0.f, qe = 0.f, qf = 0.f;
+    static __device__ __forceinline__ float two_sum(float &a, float x) {  // a += x, returns the rounding error
+        const float t = __fadd_rn(a, x), z = __fsub_rn(t, a);
+        const float e = __fadd_rn(__fsub_rn(a, __fsub_rn(t, z)), __fsub_rn(x, z));
+        a = t;
+        return e;
+    }
+    __device__ __forceinline__ void add(float x) {
+        se = __fadd_rn(se, two_sum(s, x));
+        const float p = __fmul_rn(x, x);
+        const float e = two_sum(q, p);
+        qf = __fadd_rn(qf, two_sum(qe, e));
+        qf = __fadd_rn(qf, two_sum(qe, __fmaf_rn(x, x, -p)));
+    }
+    __device__ __forceinline__ double sum() const { return static_cast<double>(s) + static_cast<double>(se); }
+    __device__ __forceinline__ double squares() const {
+        return static_cast<double>(q) + (static_cast<double>(qe) + static_cast<double>(qf));
+    }
+};
 
 // Packed nibble k -> (real, imag) = codes - 2.  A 2-bit code c placed in the
 // mantissa of 1.5 * 2^23 gives the float 12582912 + c exactly; subtracting

@@ -20,8 +20,8 @@ struct sdbe_resampler {
     int64_t max_snaps = 0;
     uint32_t *spec = nullptr;     // [2][max_snaps][2048] packed spectra
     int64_t spec_pol_stride = 0;  // words
-    uint32_t *bitmap = nullptr;   // [max_frames][64]
-    int32_t *counts = nullptr;    // [max_frames] per-frame packets, then [1] rejected
+    int32_t *counts = nullptr;    // [max_frames] per-frame packets, then [1] rejected; then, 256-byte aligned,
+    uint32_t *bitmap = nullptr;   // [max_frames][64] (the same allocation)
     float *ts = nullptr;          // [2][wave*143*32768] stage-A time series
     int64_t ts_pol_stride = 0;
     float *fout = nullptr;        // [2][128*32768] first-batch floats
@@ -285,7 +285,7 @@ int fft_chain(sdbe_resampler *h, const uint32_t *spec, int64_t spec_pol_stride, 
         o.fout_pol_stride = static_cast<int64_t>(kChunks) * kNC;
         o.partials = h->partials;
         SDBE_CK(h, launch_resample(1, h->ts, h->ts_pol_stride, h->skip, kChunks, 2, o, h->tw, st));
-        SDBE_CK(h, launch_finalize_thresholds(h->partials, kChunks, h->cfg.pol1_uses_pol0_threshold, h->thr, st));
+        SDBE_CK(h, launch_finalize_thresholds(h->partials, h->cfg.pol1_uses_pol0_threshold, h->thr, st));
         SDBE_CK(h, launch_quantize_chunks(h->fout, static_cast<int64_t>(kChunks) * kNC, kChunks, h->thr, tgt.base,
                                           tgt.pol_stride, tgt.pkt_stride, tgt.payload_off, 0, st));
         h->thresholds_set = true;

@@ -577,6 +577,15 @@ __global__ void __launch_bounds__(kNTA, 1) k_swarm_c2r(const __grid_constant__ S
     __shared__ PipeA P;
     TabsA T = tabs_a_at(sm + 3 * kBlkA);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t n_items = S.n_items;
+    const int64_t G = gridDim.x;
+    auto fetch = [&](int64_t item, int buf) {  // one thread
+        const SegA &g = S.s[seg_of(S, item)];
+        const int64_t local = item - g.item0;
+        const int64_t pol = local >= g.n_snaps, s = local - pol * g.n_snaps;  // n_pols <= 2: no division
+        tc5::bulk_g2s(sp + buf * kGroups, g.spec + pol * g.spec_pol_stride + (g.snap0 + s) * kGroups,
+                      kGroups * sizeof(uint32_t), &P.full[buf]);
+    };
     if (threadIdx.x == 0) {
         tc5::mbar_init(&P.full[0], 1);
         tc5::mbar_init(&P.full[1], 1);
@@ -584,6 +593,9 @@ __global__ void __launch_bounds__(kNTA, 1) k_swarm_c2r(const __grid_constant__ S
         tc5::mbar_init(&P.second, kNTA / 32);
         tc5::fence_mbar_init();
         P.err = 0;
+        // the first spectra on their way while the tables load
+        if (blockIdx.x < n_items) fetch(blockIdx.x, 0);
+        if (blockIdx.x + G < n_items) fetch(blockIdx.x + G, 1);
     }
     if (warp == 0) tc5::tmem_alloc(&P.tmem, kColsA);
     load_tabs_a(T, tw);
@@ -603,15 +615,6 @@ __global__ void __launch_bounds__(kNTA, 1) k_swarm_c2r(const __grid_constant__ S
     __syncthreads();  // the four warps of a quarter read one table
     tc5::fence_after();
     const LastTw lt = last_tw(T);  // once per CTA
-    const int64_t n_items = S.n_items;
-    const int64_t G = gridDim.x;
-    auto fetch = [&](int64_t item, int buf) {  // one thread
-        const SegA &g = S.s[seg_of(S, item)];
-        const int64_t local = item - g.item0;
-        const int64_t pol = local >= g.n_snaps, s = local - pol * g.n_snaps;  // n_pols <= 2: no division
-        tc5::bulk_g2s(sp + buf * kGroups, g.spec + pol * g.spec_pol_stride + (g.snap0 + s) * kGroups,
-                      kGroups * sizeof(uint32_t), &P.full[buf]);
-    };
     auto wait = [&](uint64_t *bar, uint32_t parity) { tc5::wait_or_flag(bar, parity, &P.err); };
     // Input columns of the k-th item (its spectrum in buffer k & 1), DFT-32,
     // parked.  The first pass takes Z[col + 512 r] from the packed bins X[k]
@@ -633,10 +636,6 @@ __global__ void __launch_bounds__(kNTA, 1) k_swarm_c2r(const __grid_constant__ S
         tc5::tmem_park<32>(park, v);
     };
     int64_t item = blockIdx.x;
-    if (threadIdx.x == 0) {
-        if (item < n_items) fetch(item, 0);
-        if (item + G < n_items) fetch(item + G, 1);
-    }
     if (item < n_items) input(0);
     float2 *first = sm, *second = sm + kBlkA, *spare = sm + 2 * kBlkA;
     for (uint32_t k = 0; item < n_items; item += G, ++k) {
@@ -753,37 +752,6 @@ __global__ void __launch_bounds__(kNTB, 1) k_resample(const __grid_constant__ Se
         tc5::fence_mbar_init();
         P.err = 0;
     }
-    if (warp == 0) tc5::tmem_alloc(&P.tmem, kColsB);
-    load_tabs_a(TA, tw);
-    load_tabs_b(TB, tw);
-    // the inverse's first-pass column: warp w takes those of sub-transform w,
-    // so its first two passes need no barrier but the warp's own
-    const int sub = warp, col = sub + 16 * lane;
-    const float2 wc = conjf2(__ldg(tw.w32768 + col));  // W_32768^-col
-    tc5::fence_before();
-    __syncthreads();  // tables loaded, barriers and tensor memory ready
-    tc5::fence_after();
-    const uint32_t quarter = P.tmem + (static_cast<uint32_t>(warp & 3) << 21);
-    const uint32_t tw2nd = quarter + kColTw2B, twlast = quarter + kColLast + 16u * (warp >> 2);
-    {
-        float2 w[32];
-        if (warp < 4) {
-            pass2_twiddles(TA, w);
-            tc5::tmem_park<32>(tw2nd, w);
-        }
-        const LastTw lt = last_tw(TA);
-        float2 l[8];
-        l[0] = l[7] = make_float2(0.f, 0.f);
-#pragma unroll
-        for (int j = 1; j < 4; ++j) {
-            l[j] = lt.S0[j];
-            l[3 + j] = lt.A0[j];
-        }
-        tc5::tmem_park<8>(twlast, l);
-    }
-    tc5::fence_before();
-    __syncthreads();  // the four warps of a quarter read one table
-    tc5::fence_after();
     const int64_t n_items = S.n_items, G = gridDim.x;
     auto wait = [&](uint64_t *bar, uint32_t parity) { tc5::wait_or_flag(bar, parity, &P.err); };
     auto arrive = [&](uint64_t *bar) {
@@ -819,6 +787,39 @@ __global__ void __launch_bounds__(kNTB, 1) k_resample(const __grid_constant__ Se
         }
         tc5::cp_async_commit();
     };
+    int64_t item = blockIdx.x;
+    if (item < n_items) fetch(src_of(item), 0);  // on its way while the tables load
+    if (warp == 0) tc5::tmem_alloc(&P.tmem, kColsB);
+    load_tabs_a(TA, tw);
+    load_tabs_b(TB, tw);
+    // the inverse's first-pass column: warp w takes those of sub-transform w,
+    // so its first two passes need no barrier but the warp's own
+    const int sub = warp, col = sub + 16 * lane;
+    const float2 wc = conjf2(__ldg(tw.w32768 + col));  // W_32768^-col
+    tc5::fence_before();
+    __syncthreads();  // tables loaded, barriers and tensor memory ready
+    tc5::fence_after();
+    const uint32_t quarter = P.tmem + (static_cast<uint32_t>(warp & 3) << 21);
+    const uint32_t tw2nd = quarter + kColTw2B, twlast = quarter + kColLast + 16u * (warp >> 2);
+    {
+        float2 w[32];
+        if (warp < 4) {
+            pass2_twiddles(TA, w);
+            tc5::tmem_park<32>(tw2nd, w);
+        }
+        const LastTw lt = last_tw(TA);
+        float2 l[8];
+        l[0] = l[7] = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int j = 1; j < 4; ++j) {
+            l[j] = lt.S0[j];
+            l[3 + j] = lt.A0[j];
+        }
+        tc5::tmem_park<8>(twlast, l);
+    }
+    tc5::fence_before();
+    __syncthreads();  // the four warps of a quarter read one table
+    tc5::fence_after();
     // Round r of the first pass from the stage, parked; then the next fetch.
     auto first_pass = [&](int r, const float2 *znext, int rnext) {
         tc5::cp_async_wait_all();
@@ -834,13 +835,23 @@ __global__ void __launch_bounds__(kNTB, 1) k_resample(const __grid_constant__ Se
         team_sync();  // the stage has been read
         if (znext) fetch(znext, rnext);
     };
-    int64_t item = blockIdx.x;
     if (item < n_items) {
-        const float2 *z = src_of(item), *zn = item + G < n_items ? src_of(item + G) : nullptr;
-        fetch(z, 0);
-        first_pass(0, z, 1);
-        first_pass(1, z, 2);
-        first_pass(2, zn, 0);
+        // rounds 1 and 2 of the first chunk straight to registers, beside round 0
+        const float2 *z = src_of(item);
+        float2 early[2][16];
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+                early[h][i] = t1 < 13 && m0 + 4 * (h + 1) < 11 ? __ldg(z + 8 * (m0 + 4 * (h + 1) + 11 * t1) + c1 + 1144 * i)
+                                                               : make_float2(0.f, 0.f);
+        first_pass(0, item + G < n_items ? src_of(item + G) : nullptr, 0);
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+            if (m0 + 4 * (h + 1) < 11) {
+                dft<16, false>(early[h]);
+                tc5::tmem_park<16>(quarter + kColRound + 96u * (warp >> 2) + 32u * (h + 1), early[h]);
+            }
     }
     for (uint32_t k = 0; item < n_items; item += G, ++k) {
         const SegB &g = S.s[seg_of(S, item)];
@@ -990,24 +1001,24 @@ __global__ void __launch_bounds__(kNTB, 1) k_resample(const __grid_constant__ Se
             }
         } else {
             float2 *fo = reinterpret_cast<float2 *>(o.fout + pol * o.fout_pol_stride + c * kNC);
-            double s1 = 0.0, s2 = 0.0;
+            Moments2 mo;
             auto epi = [&](int jj, const float2 *u) {
 #pragma unroll
                 for (int r = 0; r < 16; ++r) {
                     fo[jj + 1024 * r] = u[r];
                     if constexpr (MODE == 1) {
-                        const double a = u[r].x, b = u[r].y;
-                        s1 += a + b;
-                        s2 += a * a + b * b;
+                        mo.add(u[r].x);
+                        mo.add(u[r].y);
                     }
                 }
             };
             inverse(epi);
             if constexpr (MODE == 1) {
+                double s1 = mo.sum(), s2 = mo.squares();
                 block_sum2(s1, s2, red);
                 if (tid == 0) {
                     const double n = static_cast<double>(kNC);
-                    const double mean = s1 / n;
+                    const double mean = s1 * (1.0 / kNC);  // a power of two: exact
                     double *pp = o.partials + (static_cast<int64_t>(pol) * n_chunks + c) * 3;
                     pp[0] = n;
                     pp[1] = mean;
@@ -1083,40 +1094,39 @@ __global__ void __launch_bounds__(kNTB, 1)
 }
 
 // ---------------------------------------------------------------------------
-// Threshold from the per-chunk partials: Chan's merge in FP64, in chunk order
-// (deterministic).  thr_state: [0..1] effective threshold, [2..3] effective
-// offset, [4..5] own threshold, [6..7] own offset.
 struct Moments {
     double n, mean, m2;
 };
 
-// Chan et al. pairwise merge of (n, mean, M2).
-__device__ __forceinline__ Moments merge_moments(Moments a, Moments b) {
-    const double n = a.n + b.n;
-    if (n == 0.0) return a;
+// Chan et al. pairwise merge of (n, mean, M2) for equal counts.
+__device__ __forceinline__ Moments merge_equal(Moments a, Moments b) {
     const double delta = b.mean - a.mean;
-    return Moments{n, a.mean + delta * b.n / n, a.m2 + b.m2 + delta * delta * a.n * b.n / n};
+    return Moments{a.n + b.n, a.mean + 0.5 * delta, a.m2 + b.m2 + delta * delta * (0.5 * a.n)};
 }
 
 // Threshold from the per-chunk partials, FP64, one warp per pol: each lane
-// merges its chunks in order, then a fixed butterfly tree merges the lanes
+// merges its four chunks, then a fixed butterfly tree merges the lanes
 // (deterministic).  thr_state: [0..1] effective threshold, [2..3] effective
 // offset, [4..5] own threshold, [6..7] own offset.
-__global__ void k_finalize_thresholds(const double *__restrict__ partials, int n_chunks, int pol1_uses_pol0,
+__global__ void k_finalize_thresholds(const double *__restrict__ partials, int pol1_uses_pol0,
                                       float *__restrict__ thr_state) {
     __shared__ float th_s[2], off_s[2];
     const int pol = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (pol < 2) {
-        Moments m{0.0, 0.0, 0.0};
-        for (int c = lane; c < n_chunks; c += 32) {
-            const double *pp = partials + (static_cast<int64_t>(pol) * n_chunks + c) * 3;
-            m = merge_moments(m, Moments{pp[0], pp[1], pp[2]});
-        }
+        // pairs of equal counts (every chunk has kNC samples): the merge's
+        // n_b / n is 1/2 and its n_a n_b / n is n_a / 2, no division (FP64
+        // divisions, 18 of them, took 9 us)
+        static_assert(kChunks == 128, "four chunks a lane");
+        auto at = [&](int c) {
+            const double *pp = partials + (static_cast<int64_t>(pol) * kChunks + c) * 3;
+            return Moments{pp[0], pp[1], pp[2]};
+        };
+        Moments m = merge_equal(merge_equal(at(lane), at(lane + 32)), merge_equal(at(lane + 64), at(lane + 96)));
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             Moments other{__shfl_xor_sync(0xffffffffu, m.n, o), __shfl_xor_sync(0xffffffffu, m.mean, o),
                           __shfl_xor_sync(0xffffffffu, m.m2, o)};
-            m = (lane & o) ? merge_moments(other, m) : merge_moments(m, other);
+            m = (lane & o) ? merge_equal(other, m) : merge_equal(m, other);
         }
         if (lane == 0) {
             th_s[pol] = static_cast<float>(sqrt(m.m2 / (m.n - 1.0)));
@@ -1406,9 +1416,9 @@ cudaError_t launch_window_update(const WinUpds &U, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_finalize_thresholds(const double *partials, int n_chunks, int pol1_uses_pol0, float *thr_state,
+cudaError_t launch_finalize_thresholds(const double *partials, int pol1_uses_pol0, float *thr_state,
                                        cudaStream_t st) {
-    k_finalize_thresholds<<<1, 64, 0, st>>>(partials, n_chunks, pol1_uses_pol0, thr_state);
+    k_finalize_thresholds<<<1, 64, 0, st>>>(partials, pol1_uses_pol0, thr_state);
     return cudaGetLastError();
 }
 

@@ -637,15 +637,12 @@ __global__ void k_tc_chunk_stats(const float *__restrict__ y, int64_t y_pol_stri
     __shared__ double red[64];
     const int pol = blockIdx.y, c = blockIdx.x;
     const float *src = y + pol * y_pol_stride + static_cast<int64_t>(c) * kNC;
-    double s1 = 0.0, s2 = 0.0;
-    for (int i = threadIdx.x; i < kNC; i += blockDim.x) {
-        const double v = src[i];
-        s1 += v;
-        s2 += v * v;
-    }
+    Moments2 mo;
+    for (int i = threadIdx.x; i < kNC; i += blockDim.x) mo.add(src[i]);
+    double s1 = mo.sum(), s2 = mo.squares();
     block_sum2(s1, s2, red);
     if (threadIdx.x == 0) {
-        const double n = static_cast<double>(kNC), mean = s1 / n;
+        const double n = static_cast<double>(kNC), mean = s1 * (1.0 / kNC);  // a power of two: exact
         double *pp = partials + (static_cast<int64_t>(pol) * n_chunks + c) * 3;
         pp[0] = n;
         pp[1] = mean;
@@ -810,7 +807,7 @@ int tc_wave_multi(const std::vector<TcWaveItem> &w, bool first, cudaStream_t st)
         if (first) {
             k_tc_chunk_stats<<<dim3(kChunks, 2), 256, 0, st>>>(yf, chunks * kNC, kChunks, h->partials);
             SDBE_CK(h, cudaGetLastError());
-            SDBE_CK(h, launch_finalize_thresholds(h->partials, kChunks, h->cfg.pol1_uses_pol0_threshold, h->thr, st));
+            SDBE_CK(h, launch_finalize_thresholds(h->partials, h->cfg.pol1_uses_pol0_threshold, h->thr, st));
             h->thresholds_set = true;
             h->launches += 2;
         }

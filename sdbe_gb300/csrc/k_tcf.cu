@@ -751,7 +751,7 @@ __device__ __forceinline__ void inv_phase(const ArgsInv &a, const Sched sc, uint
         // z[m], m = k1 + 32 k2 + 1024 k3, = samples (2m, 2m + 1); a warp covers 32
         // consecutive m.
         float f1 = 0.f, f2 = 0.f;  // OUT_QUANT_SUMS: this thread's sums over the chunk (scaled values)
-        double d1 = 0.0, d2 = 0.0; // OUT_FLOAT_MOMENTS
+        Moments2 mo;               // OUT_FLOAT_MOMENTS
         auto epi3 = [&](int j, const SegInv &s, int64_t pol, int64_t loc) {
             const int r = 128 * j + 32 * q + lane;
             uint32_t r0[16], r1[16];
@@ -777,8 +777,8 @@ __device__ __forceinline__ void inv_phase(const ArgsInv &a, const Sched sc, uint
                     const float2 x = make_float2(kUnscaleC * v[i].x, kUnscaleC * v[i].y);
                     __stcs(fo + r + 1024 * i, x);
                     if constexpr (OUT == OUT_FLOAT_MOMENTS) {
-                        d1 += static_cast<double>(x.x) + static_cast<double>(x.y);
-                        d2 += static_cast<double>(x.x) * x.x + static_cast<double>(x.y) * x.y;
+                        mo.add(x.x);
+                        mo.add(x.y);
                     }
                 }
             } else {
@@ -819,8 +819,8 @@ __device__ __forceinline__ void inv_phase(const ArgsInv &a, const Sched sc, uint
                 if (s.o.partials == nullptr) return;
                 double s1, s2;
                 if constexpr (OUT == OUT_FLOAT_MOMENTS) {
-                    s1 = warp_sum(d1);
-                    s2 = warp_sum(d2);
+                    s1 = warp_sum(mo.sum());
+                    s2 = warp_sum(mo.squares());
                 } else {  // sums of the scaled values: x 2^21 and x 2^42 (exact)
                     s1 = static_cast<double>(warp_sum_f(f1)) * kUnscaleC;
                     s2 = static_cast<double>(warp_sum_f(f2)) * kUnscaleC * kUnscaleC;
@@ -840,15 +840,16 @@ __device__ __forceinline__ void inv_phase(const ArgsInv &a, const Sched sc, uint
                     const double nn = static_cast<double>(kNC);
                     pp[0] = nn;
                     if constexpr (OUT == OUT_FLOAT_MOMENTS) {
-                        pp[1] = t1 / nn;
-                        pp[2] = t2 - t1 * (t1 / nn);
+                        const double mean = t1 * (1.0 / kNC);  // a power of two: exact
+                        pp[1] = mean;
+                        pp[2] = t2 - t1 * mean;
                     } else {
                         pp[1] = t1;
                         pp[2] = t2;
                     }
                 }
                 team_sync();  // red reusable
-                d1 = d2 = 0.0;
+                mo = Moments2{};
                 f1 = f2 = 0.f;
             }
         };
@@ -1817,7 +1818,7 @@ int tcf_wave_multi(const std::vector<TcWaveItem> &w, bool first, cudaStream_t st
     for (const auto &it : w) {
         sdbe_resampler *h = it.h;
         if (first) {
-            SDBE_CK(h, launch_finalize_thresholds(h->partials, kChunks, h->cfg.pol1_uses_pol0_threshold, h->thr, st));
+            SDBE_CK(h, launch_finalize_thresholds(h->partials, h->cfg.pol1_uses_pol0_threshold, h->thr, st));
             const PayloadTarget &t = it.tgt;
             SDBE_CK(h, launch_quantize_chunks(h->fout, static_cast<int64_t>(kChunks) * kNC, kChunks, h->thr, t.base,
                                               t.pol_stride, t.pkt_stride, t.payload_off, it.b0 * kChunks, st));

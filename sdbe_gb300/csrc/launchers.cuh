@@ -77,7 +77,7 @@ cudaError_t launch_resample(int, const float *, int64_t, int, int64_t, int, cons
                             cudaStream_t);
 cudaError_t launch_swarm_r2c(const float *, int64_t, void *, const Twiddles &, cudaStream_t);
 cudaError_t launch_r2dbe_c2r(const void *, int64_t, int64_t, int, float *, const Twiddles &, cudaStream_t);
-cudaError_t launch_finalize_thresholds(const double *, int, int, float *, cudaStream_t);
+cudaError_t launch_finalize_thresholds(const double *, int, float *, cudaStream_t);
 struct WinUpd {  // one handle's windowed-threshold step after a wave
     const double *partials;  // [2][nb*128][3]
     double *ring;            // [2][W][3]
