@@ -69,6 +69,9 @@ struct sdbe_resampler {
     int64_t ipfb_y_bytes = 0;
     uint8_t *ipfb_scr = nullptr;  // factors [nblock][ntap][32768] f64
     int64_t ipfb_scr_bytes = 0;
+    int64_t ipfb_rows = 0;        // rows of the kept factor in ipfb_scr (of ipfb_ntap taps)
+    uint8_t *ipfb_v = nullptr;    // substituted values [nblock][32768] f64, with a kept factor
+    int64_t ipfb_v_bytes = 0;
     uint8_t *pol_scr = nullptr;   // group assembly on the device: state, result, bins, codes
     int64_t pol_scr_bytes = 0;
     int64_t ing_last_n = 0;       // packets of the last sdbe_ingest batch (their flags in ing_accept)

@@ -19,9 +19,17 @@
 // but one per row) and streamed to scratch with the forward-substituted
 // values; the backward sweep reads them once, and emits x_{m+ntap-1} as soon
 // as z_m is known (the projection P^T z fused in).
+//
+// The factor depends on ntap and the row only, not on the spectra, and row m
+// is the same for any number of blocks above m.  FP64 instructions (64 cycles
+// a warp here) bound the solve, and forming the factor anew was two thirds of
+// them, so the handle keeps it, as it keeps the window's table: k_ipfb_factor
+// forms it once for the largest call so far (up to kPlanBlocks rows), and
+// k_ipfb_apply does the two substitutions.
 #include <cuda_runtime.h>
 
 #include <cmath>
+#include <type_traits>
 #include <vector>
 
 #include "handle.cuh"
@@ -125,6 +133,147 @@ __global__ void __launch_bounds__(128) k_ipfb_solve(const float *__restrict__ y,
     }
 }
 
+// fac layout: [nblock][NT][L]: entries 0..NT-2 = L[m][m-1-k], entry NT-1 = 1/d_m.
+template <int NT>
+__global__ void __launch_bounds__(128) k_ipfb_factor(int64_t nblock, const double *__restrict__ tab,
+                                                     double *__restrict__ fac) {
+    constexpr int B = NT - 1;
+    constexpr int L = kNA;
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    double a[NT];
+#pragma unroll
+    for (int d = 0; d < NT; ++d) a[d] = tab[d * L + p];
+    double pl[B][B], pd[B], pdi[B];  // as in k_ipfb_solve
+#pragma unroll
+    for (int k = 0; k < B; ++k) {
+        pd[k] = 1.0;
+        pdi[k] = 0.0;
+#pragma unroll
+        for (int q = 0; q < B; ++q) pl[k][q] = 0.0;
+    }
+    for (int64_t m = 0; m < nblock; ++m) {
+        double l[B];
+#pragma unroll
+        for (int k = B; k >= 1; --k) {
+            double s = a[k];
+#pragma unroll
+            for (int q = k + 1; q <= B; ++q) s -= l[q - 1] * pd[q - 1] * pl[k - 1][q - k - 1];
+            l[k - 1] = m - k >= 0 ? s * pdi[k - 1] : 0.0;
+        }
+        double dm = a[0];
+#pragma unroll
+        for (int k = 1; k <= B; ++k) dm -= l[k - 1] * l[k - 1] * pd[k - 1];
+        const double dinv = 1.0 / dm;
+        double *row = fac + m * NT * L + p;
+#pragma unroll
+        for (int k = 0; k < B; ++k) row[k * L] = l[k];
+        row[B * L] = dinv;
+#pragma unroll
+        for (int k = B - 1; k >= 1; --k) {
+            pd[k] = pd[k - 1];
+            pdi[k] = pdi[k - 1];
+#pragma unroll
+            for (int q = 0; q < B; ++q) pl[k][q] = pl[k - 1][q];
+        }
+        pd[0] = dm;
+        pdi[0] = dinv;
+#pragma unroll
+        for (int q = 0; q < B; ++q) pl[0][q] = l[q];
+    }
+}
+
+// y / 32768 in FP64, exactly; the conversion by integer operations (a
+// conversion instruction takes as long as an FP64 one) but for zeros,
+// denormals, infinities and NaN.
+__device__ __forceinline__ double scaled_f64(float y) {
+    const uint32_t u = __float_as_uint(y), e = (u >> 23) & 255u;
+    if (e == 0u || e == 255u) return static_cast<double>(y) * (1.0 / kNA);
+    const uint32_t hi = (u & 0x80000000u) | (((u & 0x7FFFFFFFu) >> 3) + ((896u - 15u) << 20));
+    return __hiloint2double(static_cast<int>(hi), static_cast<int>(u << 29));
+}
+
+// Forward and backward substitution with a kept factor; v: [nblock][L] scratch.
+template <int NT>
+__global__ void __launch_bounds__(64) k_ipfb_apply(const float *__restrict__ y, int64_t nblock,
+                                                   const double *__restrict__ tab, const double *__restrict__ fac,
+                                                   double *__restrict__ v, float *__restrict__ out) {
+    static_assert(kNA == 1 << 15, "scaled_f64 divides by 2^15");
+    constexpr int B = NT - 1;
+    constexpr int L = kNA;
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    double w[NT];
+#pragma unroll
+    for (int d = 0; d < NT; ++d) w[d] = tab[(NT + d) * L + p];
+    double pw[B];
+#pragma unroll
+    for (int k = 0; k < B; ++k) pw[k] = 0.0;
+    // row m + 1 is loaded while row m is worked on
+    double f[NT];
+    float ym = __ldg(y + p);
+#pragma unroll
+    for (int k = 0; k < NT; ++k) f[k] = __ldg(fac + k * L + p);
+    for (int64_t m = 0; m < nblock; ++m) {
+        double wm = scaled_f64(ym), l[NT];
+#pragma unroll
+        for (int k = 0; k < NT; ++k) l[k] = f[k];
+        if (m + 1 < nblock) {
+            ym = __ldg(y + (m + 1) * L + p);
+#pragma unroll
+            for (int k = 0; k < NT; ++k) f[k] = __ldg(fac + ((m + 1) * NT + k) * L + p);
+        }
+#pragma unroll
+        for (int k = 1; k <= B; ++k) wm -= l[k - 1] * pw[k - 1];
+        v[m * L + p] = wm * l[B];
+#pragma unroll
+        for (int k = B - 1; k >= 1; --k) pw[k] = pw[k - 1];
+        pw[0] = wm;
+    }
+    double nl[B][B], nz[B];  // as in k_ipfb_solve
+#pragma unroll
+    for (int k = 0; k < B; ++k) {
+        nz[k] = 0.0;
+#pragma unroll
+        for (int q = 0; q < B; ++q) nl[k][q] = 0.0;
+    }
+    double vm = v[(nblock - 1) * L + p];
+#pragma unroll
+    for (int k = 0; k < B; ++k) f[k] = __ldg(fac + ((nblock - 1) * NT + k) * L + p);
+    for (int64_t m = nblock - 1; m >= 0; --m) {
+        double z = vm, l[B];
+#pragma unroll
+        for (int k = 0; k < B; ++k) l[k] = f[k];
+        if (m > 0) {
+            vm = v[(m - 1) * L + p];
+#pragma unroll
+            for (int k = 0; k < B; ++k) f[k] = __ldg(fac + ((m - 1) * NT + k) * L + p);
+        }
+#pragma unroll
+        for (int k = 1; k <= B; ++k) z -= nl[k - 1][k - 1] * nz[k - 1];
+        // x_{m+B} = sum_t w[t] z_{m+B-t}, t = 0..B  (z_{m..m+B} known)
+        double x = w[B] * z;
+#pragma unroll
+        for (int t = 0; t < B; ++t) x += w[t] * nz[B - 1 - t];
+        out[(m + B) * L + p] = static_cast<float>(x);
+#pragma unroll
+        for (int k = B - 1; k >= 1; --k) {
+            nz[k] = nz[k - 1];
+#pragma unroll
+            for (int q = 0; q < B; ++q) nl[k][q] = nl[k - 1][q];
+        }
+        nz[0] = z;
+#pragma unroll
+        for (int q = 0; q < B; ++q) nl[0][q] = l[q];
+    }
+    // x_j for j = B-1 .. 0: z_0..z_{B-1} are nz[0..B-1]
+#pragma unroll
+    for (int j = B - 1; j >= 0; --j) {
+        double x = 0.0;
+#pragma unroll
+        for (int t = 0; t <= j; ++t) x += w[t] * nz[j - t];
+        out[j * L + p] = static_cast<float>(x);
+    }
+}
+
 namespace {
 
 // Host table per ntap: a[d][p] (band of P P^T) and w[t][p] (P taps), FP64.
@@ -145,10 +294,39 @@ std::vector<double> ipfb_table(int ntap) {
     return tab;
 }
 
+// Calls of more blocks than this form the factor as they go (k_ipfb_solve):
+// their factor would hold over 4 GB beside the scratch, and is read from HBM.
+constexpr int64_t kPlanBlocks = 4096;
+
 template <int NT>
 cudaError_t launch_solve(const float *y, int64_t nblock, const double *tab, double *scr, float *out, cudaStream_t st) {
     k_ipfb_solve<NT><<<kNA / 128, 128, 0, st>>>(y, nblock, 1.0 / kNA, tab, scr, out);
     return cudaGetLastError();
+}
+template <int NT>
+cudaError_t launch_factor(int64_t nblock, const double *tab, double *fac, cudaStream_t st) {
+    k_ipfb_factor<NT><<<kNA / 128, 128, 0, st>>>(nblock, tab, fac);
+    return cudaGetLastError();
+}
+template <int NT>
+cudaError_t launch_apply(const float *y, int64_t nblock, const double *tab, const double *fac, double *v, float *out,
+                         cudaStream_t st) {
+    k_ipfb_apply<NT><<<kNA / 64, 64, 0, st>>>(y, nblock, tab, fac, v, out);
+    return cudaGetLastError();
+}
+
+// f(integral_constant<int, ntap>) for 2 <= ntap <= 8.
+template <class F>
+cudaError_t with_taps(int ntap, F f) {
+    switch (ntap) {
+        case 2: return f(std::integral_constant<int, 2>{});
+        case 3: return f(std::integral_constant<int, 3>{});
+        case 4: return f(std::integral_constant<int, 4>{});
+        case 5: return f(std::integral_constant<int, 5>{});
+        case 6: return f(std::integral_constant<int, 6>{});
+        case 7: return f(std::integral_constant<int, 7>{});
+        default: return f(std::integral_constant<int, 8>{});
+    }
 }
 
 }  // namespace
@@ -173,41 +351,51 @@ extern "C" int sdbe_inverse_pfb(sdbe_resampler *h, const void *spec_c64, int64_t
             h->ipfb_tab = nullptr;
             h->ipfb_ntap = 0;
         }
+        h->ipfb_rows = 0;
         SDBE_CK(h, cudaMalloc(&h->ipfb_tab, tab.size() * sizeof(double)));
         SDBE_CK(h, cudaMemcpyAsync(h->ipfb_tab, tab.data(), tab.size() * sizeof(double), cudaMemcpyHostToDevice, st));
         SDBE_CK(h, cudaStreamSynchronize(st));  // tab is freed on return
         h->ipfb_ntap = ntap;
     }
-    // scratch owned by the handle, grown to the largest call so far
+    // scratch owned by the handle, grown to the largest call so far: the factor
+    // (or, above kPlanBlocks, the factor with the substituted values) and, with
+    // a kept factor, the substituted values, which first serve the tensor-core
+    // C2R as its paired spectra (n x 16384 complex)
+    const bool plan = nblock <= kPlanBlocks;
     if (int rc = grow(h, &h->ipfb_y, &h->ipfb_y_bytes, nblock * kNA * static_cast<int64_t>(sizeof(float)),
                       "the inverse PFB scratch"))
         return rc;
-    if (int rc = grow(h, &h->ipfb_scr, &h->ipfb_scr_bytes,
-                      nblock * ntap * kNA * static_cast<int64_t>(sizeof(double)), "the inverse PFB scratch"))
-        return rc;
+    const int64_t need = nblock * ntap * kNA * static_cast<int64_t>(sizeof(double));
+    if (h->ipfb_scr_bytes < need || !plan) h->ipfb_rows = 0;  // the kept factor goes
+    if (int rc = grow(h, &h->ipfb_scr, &h->ipfb_scr_bytes, need, "the inverse PFB scratch")) return rc;
+    if (plan)
+        if (int rc = grow(h, &h->ipfb_v, &h->ipfb_v_bytes, nblock * kNA * static_cast<int64_t>(sizeof(double)),
+                          "the inverse PFB scratch"))
+            return rc;
     float *y = reinterpret_cast<float *>(h->ipfb_y);
-    double *scr = reinterpret_cast<double *>(h->ipfb_scr);
+    double *scr = reinterpret_cast<double *>(h->ipfb_scr), *v = reinterpret_cast<double *>(h->ipfb_v);
+    if (plan && h->ipfb_rows < nblock) {
+        SDBE_CK(h, cudaDeviceSynchronize());  // calls on other streams may still read the scratch
+        SDBE_CK(h, with_taps(ntap, [&](auto nt) { return launch_factor<decltype(nt)::value>(nblock, h->ipfb_tab, scr, st); }));
+        SDBE_CK(h, cudaStreamSynchronize(st));  // later calls, on any stream, find it complete
+        h->ipfb_rows = nblock;
+        h->launches += 1;
+    }
     cudaError_t e = cudaSuccess;
     if (h->cfg.precision != SDBE_PRECISION_FP32) {
-        // the pseudo time stream on the tensor cores; scr holds the paired spectra
-        // first (n x 16384 complex fits its n x ntap x 32768 doubles)
+        // the pseudo time stream on the tensor cores
         if (int rc = tc_c2r_spectra(h, static_cast<const float2 *>(spec_c64), kMA + 1, nblock,
-                                    reinterpret_cast<float2 *>(scr), y, st))
+                                    reinterpret_cast<float2 *>(plan ? v : scr), y, st))
             return rc;
     } else {
         e = launch_r2dbe_c2r(spec_c64, kMA + 1, nblock, 0, y, h->tw, st);
     }
-    if (e == cudaSuccess) {
-        switch (ntap) {
-            case 2: e = launch_solve<2>(y, nblock, h->ipfb_tab, scr, out, st); break;
-            case 3: e = launch_solve<3>(y, nblock, h->ipfb_tab, scr, out, st); break;
-            case 4: e = launch_solve<4>(y, nblock, h->ipfb_tab, scr, out, st); break;
-            case 5: e = launch_solve<5>(y, nblock, h->ipfb_tab, scr, out, st); break;
-            case 6: e = launch_solve<6>(y, nblock, h->ipfb_tab, scr, out, st); break;
-            case 7: e = launch_solve<7>(y, nblock, h->ipfb_tab, scr, out, st); break;
-            default: e = launch_solve<8>(y, nblock, h->ipfb_tab, scr, out, st); break;
-        }
-    }
+    if (e == cudaSuccess)
+        e = with_taps(ntap, [&](auto nt) {
+            constexpr int NT = decltype(nt)::value;
+            return plan ? launch_apply<NT>(y, nblock, h->ipfb_tab, scr, v, out, st)
+                        : launch_solve<NT>(y, nblock, h->ipfb_tab, scr, out, st);
+        });
     if (e != cudaSuccess) return fail(h, SDBE_ERR_CUDA, std::string("inverse_pfb: ") + cudaGetErrorString(e));
     h->launches += 2;
     return SDBE_OK;
