@@ -196,7 +196,7 @@ int sdbe_ingest(sdbe_resampler *h, const void *packets, int64_t n_packets, void 
             }
             rc = grow(h, &h->ing_batch, &h->ing_batch_bytes, n_pk * kPktBytes, "ingest batch");
             if (rc) return rc;
-            if (!h->reform_dev) SDBE_CK(h, cudaMalloc(&h->reform_dev, sizeof(sdbe_reform_state)));
+            if (!h->reform_dev) SDBE_CK(h, cudaMalloc(&h->reform_dev, kReformScratch));
             SDBE_CK(h, launch_unpack_8pac(src, n_packets, h->ing_batch, st));
             SDBE_CK(h, launch_beng_reform(h->ing_batch, n_pk, h->reform, h->reform_dev, hdr, st));
             SDBE_CK(h, cudaMemcpyAsync(&reform, h->reform_dev, sizeof(reform), cudaMemcpyDeviceToHost, st));
