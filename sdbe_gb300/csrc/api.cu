@@ -699,6 +699,7 @@ int sdbe_process(sdbe_resampler *h, const void *packets, int64_t n_packets, int3
     if (!g.ok) return fail(h, SDBE_ERR_CUDA, "cudaSetDevice failed");
     CallPlan c;
     int rc = plan_call(h, packets, n_packets, n_frames, b_zero, out, out_bytes, flags, pick(h, stream), c);
+    h->shipping = !rc && c.host_out && !c.aligned;
     if (!rc) rc = prepare_call(c);
     if (!rc && h->cfg.precision != SDBE_PRECISION_FP32) {
         rc = tc_chain(h, h->spec, h->spec_pol_stride, c.n_batches, c.pt, c.st,
@@ -707,6 +708,7 @@ int sdbe_process(sdbe_resampler *h, const void *packets, int64_t n_packets, int3
         rc = fft_chain(h, h->spec, h->spec_pol_stride, c.n_batches, c.pt, c.st,
                        [&](int64_t lo, int64_t hi) { return c.aligned ? SDBE_OK : ship_call(c, lo, hi); });
     }
+    h->shipping = false;
     if (!rc) rc = complete_call(c, result);
     return rc;
 }
@@ -743,7 +745,10 @@ int sdbe_process_multi(sdbe_resampler *const *hs, const sdbe_stream_desc *d, int
         SDBE_CK(hs[0], launch_fill_missing_segs(U, st));
         hs[0]->launches += U.blocks > 0 ? 2 : 1;
     }
-    if (int rc = fft_chain_multi(c)) return rc;
+    for (auto &ci : c) ci.h->shipping = ci.host_out && !ci.aligned;
+    const int chain_rc = fft_chain_multi(c);
+    for (auto &ci : c) ci.h->shipping = false;
+    if (chain_rc) return chain_rc;
     for (int i = 0; i < n; ++i)
         if (int rc = complete_call(c[i], results ? results + i : nullptr)) return rc;
     return SDBE_OK;
@@ -1003,13 +1008,11 @@ int sdbe_summary_stats(const float *in, int64_t n, double *out_host, void *strea
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int blocks = stats_partial_blocks(n);
     void *scr = nullptr;  // this thread's reusable scratch: the call waits for its stream below
-    SDBE_CK(nullptr, thread_scratch(static_cast<size_t>(blocks) * 2 * sizeof(double), &scr));
+    std::vector<double> hp(static_cast<size_t>(blocks) * 2 + 1);
+    SDBE_CK(nullptr, thread_scratch(hp.size() * sizeof(double), &scr));
     double *part = static_cast<double *>(scr);
-    std::vector<double> hp(static_cast<size_t>(blocks) * 2);
-    float shift = 0.f;  // the partial sums are of x - in[0]
-    cudaError_t e = launch_stats_partial(in, n, part, blocks, st);
+    cudaError_t e = launch_stats_partial(in, n, part, part + 2 * blocks, blocks, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(hp.data(), part, hp.size() * sizeof(double), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&shift, in, sizeof(float), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return fail(nullptr, SDBE_ERR_CUDA, std::string("summary_stats: ") + cudaGetErrorString(e));
     double s1 = 0.0, s2 = 0.0;
@@ -1019,7 +1022,7 @@ int sdbe_summary_stats(const float *in, int64_t n, double *out_host, void *strea
     }
     const double nn = static_cast<double>(n);
     const double dmean = s1 / nn;
-    out_host[0] = static_cast<double>(shift) + dmean;
+    out_host[0] = hp.back() + dmean;  // the partial sums are of x - in[0]
     out_host[1] = std::sqrt((s2 - s1 * dmean) / (nn - 1.0));
     return SDBE_OK;
 }

@@ -81,6 +81,7 @@ struct sdbe_resampler {
     std::vector<int32_t> g_fcount = std::vector<int32_t>(4 * 143, 0);
     sdbe_ingest_stats ing{};
     bool thresholds_set = false;
+    bool shipping = false;        // the running call's payloads go to host memory wave by wave
     int64_t carry = 0;
     int64_t stream_batch = 0;     // batches quantized since the stream started (window blocks)
     int window = 0;               // SDBE_THRESH_WINDOW: batches per window
@@ -165,6 +166,11 @@ struct PayloadTarget {
 // windowed thresholds not past the stream's next block boundary.
 inline int64_t wave_len(const sdbe_resampler *h, int64_t wave, int64_t remaining) {
     int64_t nb = remaining < wave ? remaining : wave;
+    // Payloads that leave for the host wave by wave: what the last wave ships
+    // is not behind any compute, so the last waves shrink (a wave's copy takes
+    // about a sixth of its compute).  128 batches of 143 frames in host
+    // memory: 8178 -> 7073 us with the FFT pipelines, 7617 without this.
+    if (h->shipping && remaining <= wave && remaining > 6) nb = (3 * remaining + 3) / 4;
     if (h->cfg.threshold_mode == SDBE_THRESH_WINDOW) {
         const int64_t to_block = SDBE_THRESH_BLOCK - h->stream_batch % SDBE_THRESH_BLOCK;
         if (nb > to_block) nb = to_block;

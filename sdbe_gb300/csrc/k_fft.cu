@@ -32,7 +32,6 @@ __host__ __device__ constexpr int padb(int a) { return a + (a >> 4); }
 // One of the 16 sub-transforms of the inverse 16384: 32 rows of 33 slots, and
 // one more so that 16 consecutive columns' stores land in 16 bank pairs.
 constexpr int kSub = 1057;
-constexpr int kPadA = 16 * kSub;
 constexpr int kPadB = padb(kMB) + 1;
 
 // Shared-memory twiddle tables (float2).  The per-pass tables are laid out
@@ -1269,22 +1268,31 @@ __global__ void k_quantize_flat(const float *__restrict__ in, uint32_t *__restri
 // Per-block FP64 sums for summary statistics over n floats, of the samples
 // shifted by the first one (x - in[0]): a large common offset then cancels
 // before the sums, not in the variance (the shifted-data algorithm; the
-// finalizers add in[0] back to the mean).
+// finalizers add in[0] back to the mean).  A thread's sums are unevaluated
+// FP32 ones (Shifted2): with four FP64 instructions a sample the kernel took
+// 27 us for 2^22 samples that 3 us would read.
+// shift (optional) receives in[0].
 __global__ void __launch_bounds__(256) k_stats_partial(const float *__restrict__ in, int64_t n,
-                                                       double *__restrict__ partials) {
+                                                       double *__restrict__ partials, double *__restrict__ shift) {
     __shared__ double red[64];
-    const double c = __ldg(in);
-    double s1 = 0.0, s2 = 0.0;
-    for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-         i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const double v = static_cast<double>(__ldg(in + i)) - c;
-        s1 += v;
-        s2 += v * v;
+    const float c = __ldg(in);
+    Shifted2 m;
+    const int64_t step = static_cast<int64_t>(gridDim.x) * blockDim.x;
+    int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    for (; i + 3 * step < n; i += 4 * step) {
+        float v[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v[k] = __ldg(in + i + k * step);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) m.add(v[k], c);
     }
+    for (; i < n; i += step) m.add(__ldg(in + i), c);
+    double s1 = m.sum(), s2 = m.squares();
     block_sum2(s1, s2, red);
     if (threadIdx.x == 0) {
         partials[2 * blockIdx.x] = s1;
         partials[2 * blockIdx.x + 1] = s2;
+        if (shift != nullptr && blockIdx.x == 0) *shift = static_cast<double>(c);
     }
 }
 
@@ -1442,11 +1450,12 @@ cudaError_t launch_quantize_flat(const float *in, uint32_t *out, int64_t n, floa
 
 int stats_partial_blocks(int64_t n) {
     int64_t b = (n + 255) / 256;
-    return static_cast<int>(b < 1216 ? (b < 1 ? 1 : b) : 1216);
+    return static_cast<int>(b < 304 ? (b < 1 ? 1 : b) : 304);  // two a SM: few FP64 sums at the end
 }
 
-cudaError_t launch_stats_partial(const float *in, int64_t n, double *partials, int blocks, cudaStream_t st) {
-    k_stats_partial<<<blocks, 256, 0, st>>>(in, n, partials);
+cudaError_t launch_stats_partial(const float *in, int64_t n, double *partials, double *shift, int blocks,
+                                 cudaStream_t st) {
+    k_stats_partial<<<blocks, 256, 0, st>>>(in, n, partials, shift);
     return cudaGetLastError();
 }
 

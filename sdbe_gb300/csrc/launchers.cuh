@@ -94,7 +94,7 @@ cudaError_t launch_quantize_chunks(const float *, int64_t, int64_t, const float 
                                    int64_t, int64_t, cudaStream_t);
 cudaError_t launch_quantize_flat(const float *, uint32_t *, int64_t, float, float, cudaStream_t);
 int stats_partial_blocks(int64_t);
-cudaError_t launch_stats_partial(const float *, int64_t, double *, int, cudaStream_t);
+cudaError_t launch_stats_partial(const float *, int64_t, double *, double *, int, cudaStream_t);
 cudaError_t launch_align_frames(const uint32_t *, int64_t, const uint32_t *, int64_t, int64_t, int64_t, int64_t, void *,
                                 int64_t, cudaStream_t);
 cudaError_t launch_save_leftover(const uint32_t *, int64_t, const uint32_t *, int64_t, int64_t, int64_t, int64_t, int64_t,

@@ -74,7 +74,7 @@ extern "C" int sdbe_summary_stats_noalloc(const float *in, int64_t n, double *ou
     cudaError_t e = noalloc_scratch(&scratch);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int blocks = static_cast<int>((n + kNoallocSamplesPerBlock - 1) / kNoallocSamplesPerBlock);
-    if (e == cudaSuccess) e = launch_stats_partial(in, n, scratch, blocks, st);
+    if (e == cudaSuccess) e = launch_stats_partial(in, n, scratch, nullptr, blocks, st);
     if (e == cudaSuccess) {
         k_noalloc_finalize<<<1, 32, 0, st>>>(in, blocks, n);
         e = cudaGetLastError();
