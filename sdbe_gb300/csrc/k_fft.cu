@@ -893,15 +893,16 @@ __global__ void __launch_bounds__(kNTB, 1) k_resample(const __grid_constant__ Se
         // the last forward pass with the R2C pairing: X[q], q <= 18304
         fwd_pass8<true>(sm, TB);
         arrive(&P.pass4);
-        wait(&P.pass4, k);
-        // The chunk after next, 146 KB, to L2 as nine bulk prefetches from nine threads
-        if (item + 2 * G < n_items && tid < 9) {  // 146432 B = 8 x 16384 + 15360, 16-byte aligned pieces
-            const uint32_t bytes = tid < 8 ? 16384u : static_cast<uint32_t>(kNB * 4 - 8 * 16384);
+        // The chunk after next, 146 KB, to L2 as nine bulk prefetches from nine
+        // threads of a warp that waits here for those with a third unit
+        if (warp == 12 && lane < 9 && item + 2 * G < n_items) {  // 146432 B = 8 x 16384 + 15360, 16-byte aligned pieces
+            const uint32_t bytes = lane < 8 ? 16384u : static_cast<uint32_t>(kNB * 4 - 8 * 16384);
             asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(
-                             reinterpret_cast<const char *>(src_of(item + 2 * G)) + 16384 * tid),
+                             reinterpret_cast<const char *>(src_of(item + 2 * G)) + 16384 * lane),
                          "r"(bytes)
                          : "memory");
         }
+        wait(&P.pass4, k);
         // The inverse's first pass loads Z'[j], j = col + 512 r, computed on the
         // fly by the C2R pairing of the window Y[j] = X[skip + j], j = 0..16384
         // (no pass of its own), with W_32768^-j = wc e^{2 pi i r/64} (wc per
