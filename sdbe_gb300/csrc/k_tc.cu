@@ -31,7 +31,11 @@
 namespace sdbe {
 namespace {
 
-constexpr int kTcThreads = 256;
+// 16 warps: the steps between the GEMMs (splits, twiddles, output) are three
+// quarters of a transform's time, and eight warps left the schedulers two each
+// (16 B-frames from a stream's start: 2270 -> 2210 us).
+constexpr int kTcThreads = 512;
+constexpr int kTcParts = kTcThreads / 128;  // warps per tensor-memory lane quarter: they share its columns by eights
 constexpr uint32_t kTmemCols = 512;
 constexpr int kTile = 4096;  // one [128 rows][16 k] FP16 operand tile, core-matrix order
 
@@ -230,7 +234,15 @@ struct TcGeo {
     // loaded once per CTA and read by both GEMMs
     static constexpr bool RES = N2 == 128 && NS == 2;
     static constexpr int NCOMP = NS == 3 ? 4 : 2;   // data components kept: re/im x hi/lo, or hi only
-    static constexpr int NRING = RES ? 8 : 4;       // DFT-tile buffers
+    // 16384 points with hi + lo data: both GEMMs read the same eight DFT-128
+    // stages, and the four data components (128 KB) leave room for six.  Stages
+    // 0-3 stay resident and 4-7 pass through two buffers, each loaded while the
+    // resident ones are multiplied: half the traffic, and a copy's latency (2 us
+    // under load) is exposed once a GEMM instead of at most of its K-steps
+    // (2210 -> 1973 us; a GEMM took 13-16k cycles for 6k of MMAs).
+    static constexpr bool PIN = N2 == 128 && NS == 3;
+    static constexpr int NPIN = PIN ? 4 : 0;
+    static constexpr int NRING = RES ? 8 : (PIN ? 6 : 4);  // DFT-tile buffers
     static constexpr uint32_t STAGE1 = 4 * kTile;   // bytes of a step-1 stage: DFT-128 [128 rows][16 k] x 4
     static constexpr uint32_t STAGE3 = 4 * NP * 32; // bytes of a step-3 stage: DFT-N2 [NP rows][16 k] x 4
     static constexpr uint32_t STAGE = STAGE3 > STAGE1 ? STAGE3 : STAGE1;
@@ -247,11 +259,11 @@ struct TcGeo {
 // so that an output is stored while the next step-1 GEMM runs).  Thread 0
 // issues the MMAs and the bulk copies of the DFT tiles through a ring of four
 // buffers (the tiles of K-step g+3 load while the MMAs of K-step g run; all
-// resident at 16384 points with FP16 data); warps 1-7 load the next item's
+// resident at 16384 points with FP16 data); warps 1-15 load the next item's
 // input into registers while the current item's step-3 GEMM runs, warp 0
 // (whose lane 0 issues) after it.
 //
-// Input element pairs: thread tid holds pairs i*256 + tid, i < NPAIR; pair p
+// Input element pairs: thread tid holds pairs i*512 + tid, i < NPAIR; pair p
 // is row (q % RG)*8 + (p & 7) and K columns 2kp, 2kp+1 with q = p >> 5 and
 // kp = (q / RG)*4 + ((p >> 3) & 3), so one warp's 32-bit stores cover whole
 // 128-byte core-matrix rows: no bank conflicts.  Step 2 rotates the order of
@@ -280,7 +292,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_fft(const __grid_constant_
     __shared__ int s_err;
     __shared__ float red[kTcThreads / 32];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int quarter = warp & 3, half = warp >> 2;
+    const int quarter = warp & 3, part = warp >> 2;
 
     if (tid == 0) {
         for (int b = 0; b < NRING; ++b) {
@@ -323,6 +335,15 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_fft(const __grid_constant_
         pend |= 1u << b;
         pend_g[b] = gg;
     };
+    // PIN: streamed stage hh (four a GEMM: DFT-128 stages 4-7) into buffer 4 + hh % 2.
+    uint32_t hh = 0;  // streamed stages issued to the MMAs so far
+    auto issue_stream = [&](uint32_t n) {
+        if (blockIdx.x + static_cast<int64_t>(n / 8) * gridDim.x >= a.n_items) return;  // two GEMMs an item
+        const int b = G::NPIN + (n & 1u);
+        bulk_load(aop + b * STAGE, a.f1 + (4 + (n & 3u)) * STAGE1, STAGE1, &full[b]);
+        pend |= 1u << b;
+        pend_g[b] = n;
+    };
     // One GEMM phase (thread 0), nst K-steps: step 1 (A = DFT-128 tiles from
     // the ring, B = the data in bop with K = 128) or step 3 (A = the data in
     // bop with K = NP, B = DFT-N2 tiles from the ring).
@@ -330,9 +351,11 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_fft(const __grid_constant_
         const uint32_t dr = tb + (step3 ? D3 : 0), di = dr + (step3 ? DI3 : DI1);
         const uint32_t idesc = instr_desc(128, NP, false), idesc_m = instr_desc(128, NP, true);
         for (int s = 0; s < nst; ++s, ++g) {
-            const int b = RES ? s : g % NRING;  // resident tiles: K-step s in buffer s
-            if (!RES && !err) {
-                if (mbar_wait(&full[b], (g / NRING) & 1u))
+            // resident tiles: K-step s in buffer s
+            const bool pinned = G::PIN && s < G::NPIN;
+            const int b = RES || pinned ? s : (G::PIN ? G::NPIN + static_cast<int>(hh & 1u) : g % NRING);
+            if (!RES && !pinned && !err) {
+                if (mbar_wait(&full[b], (G::PIN ? hh >> 1 : g / NRING) & 1u))
                     pend &= ~(1u << b);
                 else
                     err = true;
@@ -368,9 +391,21 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_fft(const __grid_constant_
                     }
                 }
             }
-            if (!RES) mma_commit(&empty[b]);
+            if (!RES && !pinned) mma_commit(&empty[b]);
             if (s == nst - 1) mma_commit(&done);
-            if (!RES && !err) {
+            if (G::PIN && !pinned) {
+                // streamed stage hh is with the tensor cores: hh - 1's buffer, when
+                // its MMAs are done, takes hh + 1; the GEMM's last stage also frees
+                // its own for the next GEMM
+                auto refill = [&](uint32_t freed) {
+                    if (!err && !mbar_wait(&empty[G::NPIN + (freed & 1u)], (freed >> 1) & 1u)) err = true;
+                    if (!err) issue_stream(freed + 2);
+                };
+                if (s > G::NPIN) refill(hh - 1);
+                if (s == nst - 1) refill(hh);
+                ++hh;
+            }
+            if (!RES && !G::PIN && !err) {
                 // the buffer of K-step g-1 takes K-step g+3 once those MMAs are done
                 if (g >= 1 && !mbar_wait(&empty[(g - 1) % NRING], ((g - 1) / NRING) & 1u)) err = true;
                 if (!err) issue_copy(g + NRING - 1);
@@ -392,7 +427,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_fft(const __grid_constant_
         const float2 *x = sg.in + pol * sg.in_pol_stride + loc * sg.in_stride;
 #pragma unroll
         for (int i = 0; i < NPAIR; ++i) {
-            const int q = i * 8 + warp;
+            const int q = i * (kTcThreads / 32) + warp;
             const int row = (q % RG) * 8 + (lane & 7);
             const int k = ((q / RG) * 4 + (lane >> 3)) * 2;
             xv[2 * i] = row < N2 ? __ldg(x + N2 * k + row) : make_float2(0.f, 0.f);
@@ -412,15 +447,21 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_fft(const __grid_constant_
                 else
                     err = true;
             }
+        } else if constexpr (G::PIN) {
+            arrive_expect_tx(&full[0], G::NPIN * STAGE1);
+            for (int k = 0; k < G::NPIN; ++k) bulk_copy(aop + k * STAGE, a.f1 + k * STAGE1, STAGE1, &full[0]);
+            issue_stream(0);
+            issue_stream(1);
+            if (!mbar_wait(&full[0], 0)) err = true;
         } else {
             for (int i = 0; i < NRING - 1; ++i) issue_copy(i);
         }
     }
     // y[k1 + 128 k2] = step-3 result x inv, a warp's stores 32 consecutive values
-    constexpr int HALF_OUT = NP / 2;
+    constexpr int NCH = NP / 8;  // chunks of 8 accumulator columns, part p's: p, p + kTcParts, ...
     auto store_out = [&](float2 *yo, float inv) {
         const int k1 = quarter * 32 + lane;
-        for (int c0 = half * HALF_OUT; c0 < (half + 1) * HALF_OUT; c0 += 8) {
+        for (int c0 = 8 * part; c0 < NP; c0 += 8 * kTcParts) {
             float dr[8], di[8];
             tmem_ld8x2(lane_base + D3 + c0, lane_base + D3 + DI3 + c0, dr, di);
 #pragma unroll
@@ -444,7 +485,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_fft(const __grid_constant_
         const float s1 = pow2_scale(block_max(m, red));
 #pragma unroll
         for (int i = 0; i < NPAIR; ++i) {
-            const int q = i * 8 + warp;
+            const int q = i * (kTcThreads / 32) + warp;
             const int row = (q % RG) * 8 + (lane & 7);
             const int k = ((q / RG) * 4 + (lane >> 3)) * 2;
             const uint32_t off = op_off(row, k, 128);
@@ -477,22 +518,22 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_fft(const __grid_constant_
         // every FP16 half below 2^14 without a pass for the maximum.  TMEM is
         // read GC chunks of 8 columns per wait.
         const int k1 = quarter * 32 + lane;
-        constexpr int HALF = NP / 2, NCH = HALF / 8, GC = G::RES ? 4 : 1;  // one chunk where registers are short
-        static_assert(NCH % GC == 0, "chunk groups");
+        constexpr int GC = G::RES ? 4 : 1;  // one chunk where registers are short
+        static_assert(GC == 1 || NCH % (GC * kTcParts) == 0, "chunk groups");
         constexpr float s2 = 1.f / 256.f;
         const int rot = lane >> 3;  // = (k1 >> 3) & 3
 #pragma unroll 1
-        for (int cg = 0; cg < NCH; cg += GC) {
+        for (int cg = part; cg < NCH; cg += GC * kTcParts) {
         uint32_t ur[8 * GC], ui[8 * GC];
 #pragma unroll
         for (int q = 0; q < GC; ++q) {
-            tmem_ld8_nw(lane_base + half * HALF + 8 * (cg + q), ur + 8 * q);
-            tmem_ld8_nw(lane_base + DI1 + half * HALF + 8 * (cg + q), ui + 8 * q);
+            tmem_ld8_nw(lane_base + 8 * (cg + kTcParts * q), ur + 8 * q);
+            tmem_ld8_nw(lane_base + DI1 + 8 * (cg + kTcParts * q), ui + 8 * q);
         }
         tmem_wait_tied<8 * GC>(ur, ui);
 #pragma unroll
         for (int q = 0; q < GC; ++q) {
-            const int c0 = half * HALF + 8 * (cg + q);
+            const int c0 = 8 * (cg + kTcParts * q);
             float2 v[8];
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
@@ -549,7 +590,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_fft(const __grid_constant_
     if (s_err && tid == 0) {  // a wait timed out: record it, let copies and MMAs in flight finish (bounded)
         *reinterpret_cast<volatile int *>(a.status) = 1;
         for (int b = 0; b < NRING; ++b)
-            if (pend & (1u << b)) mbar_wait(&full[b], (pend_g[b] / NRING) & 1u);
+            if (pend & (1u << b)) mbar_wait(&full[b], (G::PIN ? pend_g[b] >> 1 : pend_g[b] / NRING) & 1u);
         mma_commit(&done);
         mbar_wait(&done, done_n & 1u);
     }
