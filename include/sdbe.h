@@ -426,7 +426,10 @@ int sdbe_vdif_headers(void *frames, int64_t n_pkts, int64_t pol_stride_bytes, ui
  * P P^T solve and projection in FP64 (the systems are ill-conditioned).
  * 2 <= ntap <= 8; spec_c64 8-byte aligned.  The prototype compiles its
  * solve out (#if 0); this restates the method it sets up.  Uses handle
- * scratch of nblock*(4 + 8*ntap)*32768 bytes, allocated when a call needs
+ * scratch of nblock*(12 + 8*ntap)*32768 bytes (up to 4096 blocks; the factor
+ * of the solve is kept there for later calls of the same taps, and formed by
+ * the call that first needs it; above, nblock*(4 + 8*ntap)*32768, formed as
+ * the solve goes), allocated when a call needs
  * more than any earlier one (that growth synchronizes the device). */
 int sdbe_inverse_pfb(sdbe_resampler *h, const void *spec_c64, int64_t nblock, int32_t ntap, float *out,
                      void *stream);

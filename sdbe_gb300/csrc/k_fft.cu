@@ -45,12 +45,10 @@ constexpr int kTwA = kT32 + 2 * kT128;               // stage A tables
 constexpr int kTwB = kTwA + kT13 + kH18304 + kT128;  // stage BC tables
 constexpr size_t kSmemA = 2 * kGroups * sizeof(uint32_t) + (24 * kSub + kTwA) * sizeof(float2);
 constexpr size_t kSmemB = (kPadB + kTwB) * sizeof(float2);
-// Stage BC fits the 164 KB shared-memory carveout (with its 512-byte static
-// reduction buffer and the 1 KB reserved per block).  Above it (184 KB: the
-// 196 KB carveout) the kernel measured 1% slower, even with a radix-11
-// twiddle table that saves work, and at 208 KB (the 228 KB carveout) 9.5%
-// slower.
-static_assert(kSmemB + 512 + 1024 <= 164 * 1024, "stage BC shared memory above the 164 KB carveout");
+// The standalone R2C and C2R kernels fit the 164 KB shared-memory carveout.
+// Above it k_swarm_r2c's plain loads, as stage BC's did, have too little L1 for
+// their lines in flight (9% of stage BC at the 228 KB carveout).
+static_assert(kSmemB + 512 + 1024 <= 164 * 1024, "standalone kernels' shared memory above the 164 KB carveout");
 
 // ---- table loading --------------------------------------------------------
 struct TabsA {  // inverse-16384 tables
