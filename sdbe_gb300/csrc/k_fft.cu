@@ -63,6 +63,54 @@ __device__ __forceinline__ TabsA tabs_a_at(float2 *p) {
     return TabsA{p, p + kT32, p + kT32 + kT128};
 }
 
+// For a launch of an item or two per CTA, whose tables are a visible part of
+// it: their entries numbered through and dealt out evenly to the 512 threads,
+// every thread's loads issued before its first store.  One trip to L2 (about
+// 1.5k cycles) instead of one per table in the low warps (5.5k).  The packing
+// stage BC keeps the loops below: it measured 0.8% slower per chunk with this,
+// from registers given out differently.
+constexpr int kEntA = kT32 + 256, kEntB = kT13 + 143 + 128;
+struct TabEntry {
+    const float2 *src;
+    float2 *dst;
+};
+__device__ __forceinline__ TabEntry tab_entry_a(const TabsA &t, const Twiddles &tw, int m) {
+    if (m < kT32) {
+        const int j = m & 31, g = m >> 5;                       // g < 7: s = g + 1; else a = g - 6
+        const int e = g < 7 ? j * (g + 1) : 8 * j * (g - 6);   // exponent of W_1024
+        return {tw.w16384 + 16 * e, t.t32 + m};
+    }
+    const int q = (m - kT32) & 127;
+    return m < kT32 + 128 ? TabEntry{tw.w16384 + 128 * q, t.h16384 + tp(q)} : TabEntry{tw.w16384 + q, t.l16384 + tp(q)};
+}
+__device__ __forceinline__ TabEntry tab_entry_b(const TabsB &t, const Twiddles &tw, int m) {
+    if (m < kT13) {
+        const int r = (m >> 4) + 1, k = m & 15;
+        return {tw.w18304 + 88 * k * r, t.t13 + m};
+    }
+    const int q = m - kT13;
+    return q < 143 ? TabEntry{tw.w18304 + 128 * q, t.h18304 + tp(q)} : TabEntry{tw.w18304 + q - 143, t.l18304 + tp(q - 143)};
+}
+template <int N, class F>
+__device__ __forceinline__ void load_tabs(F entry) {
+    constexpr int R = (N + 511) / 512;
+    TabEntry e[R];
+    float2 v[R];
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        const int m = threadIdx.x + 512 * i;
+        if (m < N) {
+            e[i] = entry(m);
+            v[i] = __ldg(e[i].src);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+        if (static_cast<int>(threadIdx.x) + 512 * i < N) *e[i].dst = v[i];
+}
+__device__ __forceinline__ void load_tabs_ab(const TabsA &ta, const TabsB &tb, const Twiddles &tw) {
+    load_tabs<kEntA + kEntB>([&](int m) { return m < kEntA ? tab_entry_a(ta, tw, m) : tab_entry_b(tb, tw, m - kEntA); });
+}
 __device__ __forceinline__ void load_tabs_a(TabsA t, const Twiddles &tw) {
     for (int m = threadIdx.x; m < kT32; m += blockDim.x) {
         const int j = m & 31, g = m >> 5;                       // g < 7: s = g + 1; else a = g - 6
@@ -174,12 +222,21 @@ __device__ __forceinline__ void inv_pass2(float2 *slots, Apply apply) {
 // Last pass: jj = tid + 512 i, i = 0, 1; W_16384^(jj s) = W^(tid s) W^(512 i s).
 // at(r) is where sub-transform r's slots begin (r a compile-time index);
 // read_done() runs after this thread's last loads.
-template <class At, class Epi, class Done>
+// ROLL: a loop, its factors from constant memory (1 for i = 0) with the same
+// rounding.  A CTA's first item runs at half speed while its straight-line code
+// (100 KB of stage BC) comes from L2: with this and the R2C pass rolled and the
+// tables loaded at once, a first batch takes 82 us for 90.  The loop itself
+// costs 0.6% per chunk (17.14 for 17.02 us) once the code is there, and 3.5% in
+// stage A, so the kernels for many items don't take it.
+#define SDBE_W(N, E) {TwC<N, E>::c, TwC<N, E>::s}
+__constant__ float2 kLastStep[2][6] = {{{1.f, 0.f}, {1.f, 0.f}, {1.f, 0.f}, {1.f, 0.f}, {1.f, 0.f}, {1.f, 0.f}},
+                                       {SDBE_W(kMA, 512), SDBE_W(kMA, 1024), SDBE_W(kMA, 1536), SDBE_W(kMA, 2048),
+                                        SDBE_W(kMA, 4096), SDBE_W(kMA, 6144)}};
+template <bool ROLL, class At, class Epi, class Done>
 __device__ __forceinline__ void inv_pass3(At at, const LastTw &lt, Epi epi, Done read_done) {
     const int tid = threadIdx.x;
     const float2 *S0 = lt.S0, *A0 = lt.A0;
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
+    auto half = [&](int i, auto cst) {
         const int jj = tid + 512 * i;
         float2 u[16];
         const int o = pad(jj);
@@ -188,12 +245,20 @@ __device__ __forceinline__ void inv_pass3(At at, const LastTw &lt, Epi epi, Done
         if (i == 1) read_done();
         // W_16384^{jj r} = A[r/4] * S[r%4]
         float2 S[4], A[4];
-        S[1] = i ? mul_tc<kMA, 512, false>(S0[1]) : S0[1];
-        S[2] = i ? mul_tc<kMA, 1024, false>(S0[2]) : S0[2];
-        S[3] = i ? mul_tc<kMA, 1536, false>(S0[3]) : S0[3];
-        A[1] = i ? mul_tc<kMA, 2048, false>(A0[1]) : A0[1];
-        A[2] = i ? mul_tc<kMA, 4096, false>(A0[2]) : A0[2];
-        A[3] = i ? mul_tc<kMA, 6144, false>(A0[3]) : A0[3];
+        if constexpr (decltype(cst)::value) {
+            S[1] = i ? mul_tc<kMA, 512, false>(S0[1]) : S0[1];
+            S[2] = i ? mul_tc<kMA, 1024, false>(S0[2]) : S0[2];
+            S[3] = i ? mul_tc<kMA, 1536, false>(S0[3]) : S0[3];
+            A[1] = i ? mul_tc<kMA, 2048, false>(A0[1]) : A0[1];
+            A[2] = i ? mul_tc<kMA, 4096, false>(A0[2]) : A0[2];
+            A[3] = i ? mul_tc<kMA, 6144, false>(A0[3]) : A0[3];
+        } else {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                S[k + 1] = cmul_rn<0, 1>(S0[k + 1], kLastStep[i][k]);
+                A[k + 1] = cmul_rn<0, 0>(A0[k + 1], kLastStep[i][3 + k]);
+            }
+        }
 #pragma unroll
         for (int r = 1; r < 16; ++r) {
             const int a = r >> 2, s = r & 3;
@@ -202,10 +267,16 @@ __device__ __forceinline__ void inv_pass3(At at, const LastTw &lt, Epi epi, Done
         }
         dft<16, true>(u);
         epi(jj, u);
+    };
+    if constexpr (ROLL) {
+#pragma unroll 1
+        for (int i = 0; i < 2; ++i) half(i, std::false_type{});
+    } else {
+        half(0, std::true_type{});
+        half(1, std::true_type{});
     }
 }
 
-// f(integral_constant<int, R>) for each R: a loop over compile-time indices.
 template <int... R, class F>
 __device__ __forceinline__ void for_r(std::integer_sequence<int, R...>, F f) {
     (f(std::integral_constant<int, R>{}), ...);
@@ -266,7 +337,12 @@ __device__ __forceinline__ float2 r2c_tw(float2 wu) {
     constexpr int X = MID ? (R == 3 ? 1 : 0) : (R >= 5 ? 2 : 0), Y = MID ? (R == 3 ? 0 : 1) : (R >= 5 ? 2 : 1);
     return cmul_rn<X, Y>(wu, make_float2(TwC<16, R>::c, TwC<16, R>::s));
 }
-template <bool R2C>
+// ROLL: units in a loop (see inv_pass3); kUnitStep: W_18304^(512 i q), q = 1..4, and W_36608^(512 i).
+__constant__ float2 kUnitStep[3][5] = {
+    {{1.f, 0.f}, {1.f, 0.f}, {1.f, 0.f}, {1.f, 0.f}, {1.f, 0.f}},
+    {SDBE_W(kMB, 512), SDBE_W(kMB, 1024), SDBE_W(kMB, 1536), SDBE_W(kMB, 2048), SDBE_W(kNB, 512)},
+    {SDBE_W(kMB, 1024), SDBE_W(kMB, 2048), SDBE_W(kMB, 3072), SDBE_W(kMB, 4096), SDBE_W(kNB, 1024)}};
+template <bool R2C, bool ROLL = false>
 __device__ __forceinline__ void fwd_pass8(float2 *sm, const TabsB &T) {
     // twiddles W_18304^{k r} = A[r/4] * S[r%4]
     // butterfly k with its twiddles S[q] = W^(k q), q = 1..3, and A1 = W^(4 k)
@@ -307,19 +383,11 @@ __device__ __forceinline__ void fwd_pass8(float2 *sm, const TabsB &T) {
 #pragma unroll
         for (int q = 1; q <= 4; ++q) B[q] = tw2(T.h18304, T.l18304, tid * q);
         const float2 wt = __ldg(T.w36608 + tid);  // W_36608^tid
-        for_r(std::make_integer_sequence<int, 3>{}, [&](auto ic) {
-            constexpr int i = decltype(ic)::value;
-            const int u = tid + 512 * i;
-            if (u > K / 2) return;
-            float2 S[4];
-            S[1] = mul_tc<kMB, 512 * i, false>(B[1]);
-            S[2] = mul_tc<kMB, 1024 * i, false>(B[2]);
-            S[3] = mul_tc<kMB, 1536 * i, false>(B[3]);
-            const float2 A1 = mul_tc<kMB, 2048 * i, false>(B[4]);
+        auto unit = [&](int u, const float2 (&S)[4], float2 A1, auto wu_at) {
             float2 a[8];
             bfly8w(u, a, S, A1);
             float2 *pa = sm + padb(u);
-            const float2 wu = mul_tc<kNB, 512 * i, false>(wt);
+            const float2 wu = wu_at();
             if (u == 0) {  // q = 2288 r pairs with 2288 (8 - r); X[0], X[18304] from Z[0]
                 pa[0] = make_float2(a[0].x + a[0].y, 0.f);
                 sm[padb(kMB)] = make_float2(a[0].x - a[0].y, 0.f);
@@ -354,7 +422,29 @@ __device__ __forceinline__ void fwd_pass8(float2 *sm, const TabsB &T) {
                     pb[2431 * (7 - r)] = xmq;
                 });
             }
-        });
+        };
+        if constexpr (ROLL) {
+#pragma unroll 1
+            for (int i = 0; i < 3; ++i) {
+                const int u = tid + 512 * i;
+                if (u > K / 2) break;
+                float2 S[4];
+#pragma unroll
+                for (int q = 1; q < 4; ++q) S[q] = cmul_rn<0, 1>(B[q], kUnitStep[i][q - 1]);
+                unit(u, S, cmul_rn<0, 1>(B[4], kUnitStep[i][3]), [&] { return cmul_rn<0, 1>(wt, kUnitStep[i][4]); });
+            }
+        } else {
+            for_r(std::make_integer_sequence<int, 3>{}, [&](auto ic) {
+                constexpr int i = decltype(ic)::value;
+                const int u = tid + 512 * i;
+                if (u > K / 2) return;
+                float2 S[4];
+                S[1] = mul_tc<kMB, 512 * i, false>(B[1]);
+                S[2] = mul_tc<kMB, 1024 * i, false>(B[2]);
+                S[3] = mul_tc<kMB, 1536 * i, false>(B[3]);
+                unit(u, S, mul_tc<kMB, 2048 * i, false>(B[4]), [&] { return mul_tc<kNB, 512 * i, false>(wt); });
+            });
+        }
     }
 }
 
@@ -595,7 +685,7 @@ __global__ void __launch_bounds__(kNTA, 1) k_swarm_c2r(const __grid_constant__ S
         if (blockIdx.x + G < n_items) fetch(blockIdx.x + G, 1);
     }
     if (warp == 0) tc5::tmem_alloc(&P.tmem, kColsA);
-    load_tabs_a(T, tw);
+    load_tabs<kEntA>([&](int m) { return tab_entry_a(T, tw, m); });
     const int col = c2r_col(c2r_slot(threadIdx.x)), sub = c2r_sub(threadIdx.x);
     const float2 wc = conjf2(__ldg(tw.w32768 + col));  // W_32768^-col
     tc5::fence_before();
@@ -665,7 +755,7 @@ __global__ void __launch_bounds__(kNTA, 1) k_swarm_c2r(const __grid_constant__ S
         const int64_t local = item - g.item0;
         const int64_t pol = local >= g.n_snaps, s = local - pol * g.n_snaps;
         float2 *dst = reinterpret_cast<float2 *>(g.out + pol * g.out_pol_stride + s * kNA);
-        inv_pass3(
+        inv_pass3<false>(
             [&](int r) { return (blk_second(r) ? second : first) + kSub * blk_index(r); }, lt,
             [&](int jj, const float2 *u) {
 #pragma unroll
@@ -742,6 +832,8 @@ __global__ void __launch_bounds__(kNTB, 1) k_resample(const __grid_constant__ Se
     TabsB TB = tabs_b_at(tb, tw);
     __shared__ double red[64];
     __shared__ PipeB P;
+    // the forms with float output run a chunk or two per CTA as a rule
+    constexpr bool ROLL = MODE == 1 || MODE == 2;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (tid == 0) {
         uint64_t *bars[6] = {&P.xfree, &P.pass2, &P.pass3, &P.pass4, &P.taken, &P.inv2};
@@ -787,8 +879,12 @@ __global__ void __launch_bounds__(kNTB, 1) k_resample(const __grid_constant__ Se
     int64_t item = blockIdx.x;
     if (item < n_items) fetch(src_of(item), 0);  // on its way while the tables load
     if (warp == 0) tc5::tmem_alloc(&P.tmem, kColsB);
-    load_tabs_a(TA, tw);
-    load_tabs_b(TB, tw);
+    if constexpr (ROLL) {
+        load_tabs_ab(TA, TB, tw);
+    } else {
+        load_tabs_a(TA, tw);
+        load_tabs_b(TB, tw);
+    }
     // the inverse's first-pass column: warp w takes those of sub-transform w,
     // so its first two passes need no barrier but the warp's own
     const int sub = warp, col = sub + 16 * lane;
@@ -889,7 +985,7 @@ __global__ void __launch_bounds__(kNTB, 1) k_resample(const __grid_constant__ Se
         if (more) first_pass(1, zn, 2);
         wait(&P.pass3, k);
         // the last forward pass with the R2C pairing: X[q], q <= 18304
-        fwd_pass8<true>(sm, TB);
+        fwd_pass8<true, ROLL>(sm, TB);
         arrive(&P.pass4);
         // The chunk after next, 146 KB, to L2 as nine bulk prefetches from nine
         // threads of a warp that waits here for those with a third unit
@@ -948,7 +1044,7 @@ __global__ void __launch_bounds__(kNTB, 1) k_resample(const __grid_constant__ Se
                 }
             }
             wait(&P.inv2, k);
-            inv_pass3([&](int r) { return sm + kSub * r; }, lt, epi, [&] { arrive(&P.xfree); });
+            inv_pass3<ROLL>([&](int r) { return sm + kSub * r; }, lt, epi, [&] { arrive(&P.xfree); });
         };
         if constexpr (MODE == 0 || MODE == 3) {
             uint32_t *words = reinterpret_cast<uint32_t *>(o.out + pol * o.out_pol_stride +
@@ -1087,7 +1183,7 @@ __global__ void __launch_bounds__(kNTB, 1)
             for (int r = 1; r < 32; ++r) v[r] = cmulc(v[r], w[r]);
         });
         __syncthreads();
-        inv_pass3([&](int r) { return sm + kSub * r; }, last_tw(TA), epi, [] {});
+        inv_pass3<true>([&](int r) { return sm + kSub * r; }, last_tw(TA), epi, [] {});
     }
 }
 
