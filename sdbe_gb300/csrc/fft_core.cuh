@@ -386,12 +386,14 @@ struct Moments2 {
 struct Shifted2 {
     Moments2 m;
     double fs = 0.0, fq = 0.0;
+    bool wide = false;  // fs and fq hold something
     __device__ __forceinline__ void add(float x, float c) {
         const float dh0 = __fsub_rn(x, c);
         if (!(fabsf(dh0) < 1e12f) || (fabsf(dh0) < 1e-10f && dh0 != 0.f)) {
             const double v = static_cast<double>(x) - static_cast<double>(c);
             fs += v;
             fq += v * v;
+            wide = true;
             return;
         }
         float dh = x;
@@ -404,9 +406,57 @@ struct Shifted2 {
         f = __fadd_rn(f, __fmaf_rn(dl, dl, __fmaf_rn(2.f * dh, dl, -cr)));
         m.qf = __fadd_rn(m.qf, f);
     }
-    __device__ __forceinline__ double sum() const { return fs + m.sum(); }
-    __device__ __forceinline__ double squares() const { return fq + m.squares(); }
 };
+
+// An unevaluated sum a + b + c of FP32 values, merged across lanes and warps
+// before it is turned into FP64: the conversions and the shuffle trees of all
+// warps in FP64 took 20 instructions a warp at 76 cycles each.
+struct Sum3 {
+    float a, b, c;
+    __device__ __forceinline__ void merge(float oa, float ob, float oc) {
+        const float e = Moments2::two_sum(a, oa);
+        const float f = Moments2::two_sum(b, ob);
+        c = __fadd_rn(__fadd_rn(c, oc), __fadd_rn(f, Moments2::two_sum(b, e)));
+    }
+    template <int N>
+    __device__ __forceinline__ void merge_lanes() {  // over N lanes
+#pragma unroll
+        for (int m = N / 2; m > 0; m >>= 1) {
+            const float oa = __shfl_xor_sync(0xffffffffu, a, m), ob = __shfl_xor_sync(0xffffffffu, b, m),
+                        oc = __shfl_xor_sync(0xffffffffu, c, m);
+            merge(oa, ob, oc);
+        }
+    }
+    __device__ __forceinline__ double value() const {
+        return static_cast<double>(a) + (static_cast<double>(b) + static_cast<double>(c));
+    }
+};
+
+// The sums of m over a block of NW full warps (a power of two <= 16); result
+// valid in warp 0.  scratch: 6 * 16 floats.
+template <int NW>
+__device__ __forceinline__ void block_moments(const Moments2 &m, double &s1, double &s2, float *scratch) {
+    Sum3 s{m.s, m.se, 0.f}, q{m.q, m.qe, m.qf};
+    s.merge_lanes<32>();
+    q.merge_lanes<32>();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __syncthreads();
+    if (lane == 0) {
+        const float v[6] = {s.a, s.b, s.c, q.a, q.b, q.c};
+#pragma unroll
+        for (int k = 0; k < 6; ++k) scratch[16 * k + warp] = v[k];
+    }
+    __syncthreads();
+    if (warp == 0) {
+        const float *p = scratch + (lane & (NW - 1));
+        s = Sum3{p[0], p[16], p[32]};
+        q = Sum3{p[48], p[64], p[80]};
+        s.merge_lanes<NW>();
+        q.merge_lanes<NW>();
+        s1 = s.value();
+        s2 = q.value();
+    }
+}
 
 // Packed nibble k -> (real, imag) = codes - 2.  A 2-bit code c placed in the
 // mantissa of 1.5 * 2^23 gives the float 12582912 + c exactly; subtracting

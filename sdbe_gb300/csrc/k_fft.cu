@@ -1108,8 +1108,8 @@ __global__ void __launch_bounds__(kNTB, 1) k_resample(const __grid_constant__ Se
             };
             inverse(epi);
             if constexpr (MODE == 1) {
-                double s1 = mo.sum(), s2 = mo.squares();
-                block_sum2(s1, s2, red);
+                double s1, s2;
+                block_moments<kNTB / 32>(mo, s1, s2, reinterpret_cast<float *>(red));
                 if (tid == 0) {
                     const double n = static_cast<double>(kNC);
                     const double mean = s1 * (1.0 / kNC);  // a power of two: exact
@@ -1365,7 +1365,9 @@ __global__ void k_quantize_flat(const float *__restrict__ in, uint32_t *__restri
 // before the sums, not in the variance (the shifted-data algorithm; the
 // finalizers add in[0] back to the mean).  A thread's sums are unevaluated
 // FP32 ones (Shifted2): with four FP64 instructions a sample the kernel took
-// 27 us for 2^22 samples that 3 us would read.
+// 27 us for 2^22 samples that 3 us would read.  A batch of 1.1 million samples
+// is 14 a thread: all loaded at once, and the block's sums turned into FP64
+// once (block_moments), took another 4 us off a call.
 // shift (optional) receives in[0].
 __global__ void __launch_bounds__(256) k_stats_partial(const float *__restrict__ in, int64_t n,
                                                        double *__restrict__ partials, double *__restrict__ shift) {
@@ -1373,17 +1375,24 @@ __global__ void __launch_bounds__(256) k_stats_partial(const float *__restrict__
     const float c = __ldg(in);
     Shifted2 m;
     const int64_t step = static_cast<int64_t>(gridDim.x) * blockDim.x;
-    int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    for (; i + 3 * step < n; i += 4 * step) {
-        float v[4];
+    constexpr int U = 16;
+    for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += U * step) {
+        float v[U];
+        const int left = static_cast<int>(min(static_cast<int64_t>(U), (n - i + step - 1) / step));
 #pragma unroll
-        for (int k = 0; k < 4; ++k) v[k] = __ldg(in + i + k * step);
+        for (int k = 0; k < U; ++k)
+            if (k < left) v[k] = __ldg(in + i + k * step);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) m.add(v[k], c);
+        for (int k = 0; k < U; ++k)
+            if (k < left) m.add(v[k], c);
     }
-    for (; i < n; i += step) m.add(__ldg(in + i), c);
-    double s1 = m.sum(), s2 = m.squares();
-    block_sum2(s1, s2, red);
+    double s1, s2;
+    block_moments<8>(m.m, s1, s2, reinterpret_cast<float *>(red));
+    if (__syncthreads_or(m.wide)) {
+        block_sum2(m.fs, m.fq, red);
+        s1 += m.fs;
+        s2 += m.fq;
+    }
     if (threadIdx.x == 0) {
         partials[2 * blockIdx.x] = s1;
         partials[2 * blockIdx.x + 1] = s2;

@@ -680,8 +680,8 @@ __global__ void k_tc_chunk_stats(const float *__restrict__ y, int64_t y_pol_stri
     const float *src = y + pol * y_pol_stride + static_cast<int64_t>(c) * kNC;
     Moments2 mo;
     for (int i = threadIdx.x; i < kNC; i += blockDim.x) mo.add(src[i]);
-    double s1 = mo.sum(), s2 = mo.squares();
-    block_sum2(s1, s2, red);
+    double s1, s2;
+    block_moments<8>(mo, s1, s2, reinterpret_cast<float *>(red));
     if (threadIdx.x == 0) {
         const double n = static_cast<double>(kNC), mean = s1 * (1.0 / kNC);  // a power of two: exact
         double *pp = partials + (static_cast<int64_t>(pol) * n_chunks + c) * 3;
