@@ -182,45 +182,90 @@ __global__ void __launch_bounds__(128) k_ipfb_factor(int64_t nblock, const doubl
     }
 }
 
+// The conversions as instructions; functions, so that no FP64 instruction of
+// theirs is issued, predicated off, in the ordinary case (three of 14 a row).
+__device__ __noinline__ double scaled_f64_instr(float y) { return static_cast<double>(y) * (1.0 / kNA); }
+__device__ __noinline__ float rounded_f32_instr(double x) { return static_cast<float>(x); }
+
 // y / 32768 in FP64, exactly; the conversion by integer operations (a
 // conversion instruction takes as long as an FP64 one) but for zeros,
 // denormals, infinities and NaN.
 __device__ __forceinline__ double scaled_f64(float y) {
     const uint32_t u = __float_as_uint(y), e = (u >> 23) & 255u;
-    if (e == 0u || e == 255u) return static_cast<double>(y) * (1.0 / kNA);
+    if (e == 0u || e == 255u) return scaled_f64_instr(y);
     const uint32_t hi = (u & 0x80000000u) | (((u & 0x7FFFFFFFu) >> 3) + ((896u - 15u) << 20));
     return __hiloint2double(static_cast<int>(hi), static_cast<int>(u << 29));
 }
 
+// x in FP32, rounded to nearest even by integer operations where the result is
+// a normal number (as scaled_f64).
+__device__ __forceinline__ float rounded_f32(double x) {
+    const uint32_t hi = static_cast<uint32_t>(__double2hiint(x)), lo = static_cast<uint32_t>(__double2loint(x));
+    const uint32_t e = (hi >> 20) & 2047u;
+    if (e - 897u > 252u) return rounded_f32_instr(x);  // below FP32's normal numbers, or at its last binade or above
+    const uint32_t mag = ((hi & 0x7FFFFFFFu) - (896u << 20)) << 3 | lo >> 29;
+    const uint32_t up = (lo & 0x1FFFFFFFu) + 0x0FFFFFFFu + (mag & 1u);  // carries into bit 29 where it rounds up
+    return __uint_as_float((hi & 0x80000000u) | (mag + (up >> 29)));
+}
+
+// Rows of k_ipfb_apply in flight (a power of two): two rows 72.7, four 67.7,
+// eight 68.3, sixteen 71.8 us a call of 48 blocks, caches cold.
+constexpr int kRing = 4;
+// Asynchronous copies to shared memory that only the issuing thread reads.
+__device__ __forceinline__ void copy_async8(void *dst, const void *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void copy_async4(void *dst, const void *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void copy_wait() {  // all but the last N groups have landed
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
 // Forward and backward substitution with a kept factor; v: [nblock][L] scratch.
+// One warp per CTA, so that 1024 warps leave no sub-partition with more than
+// two.  FP64 issue (64 cycles a warp instruction, 11 for a row of four taps) is
+// the bound, if a row's values are there: four instructions of the forward
+// sweep are a fraction of a trip to DRAM, so kRing rows are on their way.  48
+// blocks, four taps: 60.8 us with one row ahead and 14 FP64 instructions a row,
+// now 38.0, of which two warps' instructions take 33.4.
 template <int NT>
-__global__ void __launch_bounds__(64) k_ipfb_apply(const float *__restrict__ y, int64_t nblock,
+__global__ void __launch_bounds__(32) k_ipfb_apply(const float *__restrict__ y, int64_t nblock,
                                                    const double *__restrict__ tab, const double *__restrict__ fac,
                                                    double *__restrict__ v, float *__restrict__ out) {
     static_assert(kNA == 1 << 15, "scaled_f64 divides by 2^15");
     constexpr int B = NT - 1;
     constexpr int L = kNA;
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ double ring[kRing][NT][32];
+    __shared__ float yring[kRing][32];
+    const int lane = threadIdx.x, p = blockIdx.x * 32 + lane;
     double w[NT];
 #pragma unroll
     for (int d = 0; d < NT; ++d) w[d] = tab[(NT + d) * L + p];
     double pw[B];
 #pragma unroll
     for (int k = 0; k < B; ++k) pw[k] = 0.0;
-    // row m + 1 is loaded while row m is worked on
-    double f[NT];
-    float ym = __ldg(y + p);
+    auto forward_row = [&](int64_t m) {
+        if (m < nblock) {
+            const int s = static_cast<int>(m) & (kRing - 1);
+            copy_async4(&yring[s][lane], y + m * L + p);
 #pragma unroll
-    for (int k = 0; k < NT; ++k) f[k] = __ldg(fac + k * L + p);
-    for (int64_t m = 0; m < nblock; ++m) {
-        double wm = scaled_f64(ym), l[NT];
-#pragma unroll
-        for (int k = 0; k < NT; ++k) l[k] = f[k];
-        if (m + 1 < nblock) {
-            ym = __ldg(y + (m + 1) * L + p);
-#pragma unroll
-            for (int k = 0; k < NT; ++k) f[k] = __ldg(fac + ((m + 1) * NT + k) * L + p);
+            for (int k = 0; k < NT; ++k) copy_async8(&ring[s][k][lane], fac + (m * NT + k) * L + p);
         }
+        copy_commit();
+    };
+    for (int i = 0; i < kRing; ++i) forward_row(i);
+    for (int64_t m = 0; m < nblock; ++m) {
+        copy_wait<kRing - 1>();
+        const int s = static_cast<int>(m) & (kRing - 1);
+        double wm = scaled_f64(yring[s][lane]), l[NT];
+#pragma unroll
+        for (int k = 0; k < NT; ++k) l[k] = ring[s][k][lane];
+        forward_row(m + kRing);
 #pragma unroll
         for (int k = 1; k <= B; ++k) wm -= l[k - 1] * pw[k - 1];
         v[m * L + p] = wm * l[B];
@@ -235,25 +280,31 @@ __global__ void __launch_bounds__(64) k_ipfb_apply(const float *__restrict__ y, 
 #pragma unroll
         for (int q = 0; q < B; ++q) nl[k][q] = 0.0;
     }
-    double vm = v[(nblock - 1) * L + p];
+    auto backward_row = [&](int64_t m) {
+        if (m >= 0) {
+            const int s = static_cast<int>(m) & (kRing - 1);
 #pragma unroll
-    for (int k = 0; k < B; ++k) f[k] = __ldg(fac + ((nblock - 1) * NT + k) * L + p);
+            for (int k = 0; k < B; ++k) copy_async8(&ring[s][k][lane], fac + (m * NT + k) * L + p);
+        }
+        copy_commit();
+    };
+    for (int i = 1; i <= kRing; ++i) backward_row(nblock - i);
+    double vm = v[(nblock - 1) * L + p];
     for (int64_t m = nblock - 1; m >= 0; --m) {
+        copy_wait<kRing - 1>();
+        const int s = static_cast<int>(m) & (kRing - 1);
         double z = vm, l[B];
 #pragma unroll
-        for (int k = 0; k < B; ++k) l[k] = f[k];
-        if (m > 0) {
-            vm = v[(m - 1) * L + p];
-#pragma unroll
-            for (int k = 0; k < B; ++k) f[k] = __ldg(fac + ((m - 1) * NT + k) * L + p);
-        }
+        for (int k = 0; k < B; ++k) l[k] = ring[s][k][lane];
+        backward_row(m - kRing);
+        if (m > 0) vm = v[(m - 1) * L + p];
 #pragma unroll
         for (int k = 1; k <= B; ++k) z -= nl[k - 1][k - 1] * nz[k - 1];
         // x_{m+B} = sum_t w[t] z_{m+B-t}, t = 0..B  (z_{m..m+B} known)
         double x = w[B] * z;
 #pragma unroll
         for (int t = 0; t < B; ++t) x += w[t] * nz[B - 1 - t];
-        out[(m + B) * L + p] = static_cast<float>(x);
+        out[(m + B) * L + p] = rounded_f32(x);
 #pragma unroll
         for (int k = B - 1; k >= 1; --k) {
             nz[k] = nz[k - 1];
@@ -311,7 +362,7 @@ cudaError_t launch_factor(int64_t nblock, const double *tab, double *fac, cudaSt
 template <int NT>
 cudaError_t launch_apply(const float *y, int64_t nblock, const double *tab, const double *fac, double *v, float *out,
                          cudaStream_t st) {
-    k_ipfb_apply<NT><<<kNA / 64, 64, 0, st>>>(y, nblock, tab, fac, v, out);
+    k_ipfb_apply<NT><<<kNA / 32, 32, 0, st>>>(y, nblock, tab, fac, v, out);
     return cudaGetLastError();
 }
 

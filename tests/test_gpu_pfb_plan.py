@@ -51,3 +51,21 @@ def test_zeros_denormals_and_large_values():
     ref = O.inverse_pfb(S.astype(np.complex128), 4)
     err = np.sqrt(np.mean((got - ref) ** 2) / np.mean(ref ** 2))
     assert err < TOL, err
+
+
+@pytest.mark.parametrize("ntap,nb", [(n, b) for n in (2, 4, 8) for b in (1, 3, 4, 5, 8)])
+@pytest.mark.parametrize("scale", [1.0, 1e-41])
+def test_rows_in_flight_and_small_results(ntap, nb, scale):
+    """Fewer, as many and more rows than are in flight at once; results among
+    FP32's normal numbers, and around the smallest of them (rounded by parts).
+    Tolerance as above, plus FP32's spacing of 2^-149 there."""
+    import __graft_entry__ as g
+
+    g.build()
+    from sdbe_gb300 import Resampler, pfb
+
+    S = (_spectra(ntap, nb, 40 + ntap) * scale).astype(np.complex64)
+    with Resampler(max_frames=1) as r:
+        got = pfb.inverse_pfb(r, S, ntap=ntap).cpu().numpy().astype(np.float64)
+    ref = O.inverse_pfb(S.astype(np.complex128), ntap)
+    assert np.sqrt(np.mean((got - ref) ** 2)) < TOL * np.sqrt(np.mean(ref ** 2)) + 2.0 ** -149
