@@ -79,7 +79,6 @@ void free_all(sdbe_resampler *h) {
     cudaFree(h->ipfb_tab);
     cudaFree(h->ipfb_y);
     cudaFree(h->ipfb_scr);
-    cudaFree(h->ipfb_v);
     cudaFree(h->wring);
     cudaFree(h->wpart);
     cudaFree(h->tc_f128);

@@ -413,18 +413,15 @@ extern "C" int sdbe_inverse_pfb(sdbe_resampler *h, const void *spec_c64, int64_t
     // a kept factor, the substituted values, which first serve the tensor-core
     // C2R as its paired spectra (n x 16384 complex)
     const bool plan = nblock <= kPlanBlocks;
-    if (int rc = grow(h, &h->ipfb_y, &h->ipfb_y_bytes, nblock * kNA * static_cast<int64_t>(sizeof(float)),
+    const int64_t v_bytes = plan ? nblock * kNA * static_cast<int64_t>(sizeof(double)) : 0;
+    if (int rc = grow(h, &h->ipfb_y, &h->ipfb_y_bytes, v_bytes + nblock * kNA * static_cast<int64_t>(sizeof(float)),
                       "the inverse PFB scratch"))
         return rc;
     const int64_t need = nblock * ntap * kNA * static_cast<int64_t>(sizeof(double));
     if (h->ipfb_scr_bytes < need || !plan) h->ipfb_rows = 0;  // the kept factor goes
     if (int rc = grow(h, &h->ipfb_scr, &h->ipfb_scr_bytes, need, "the inverse PFB scratch")) return rc;
-    if (plan)
-        if (int rc = grow(h, &h->ipfb_v, &h->ipfb_v_bytes, nblock * kNA * static_cast<int64_t>(sizeof(double)),
-                          "the inverse PFB scratch"))
-            return rc;
-    float *y = reinterpret_cast<float *>(h->ipfb_y);
-    double *scr = reinterpret_cast<double *>(h->ipfb_scr), *v = reinterpret_cast<double *>(h->ipfb_v);
+    float *y = reinterpret_cast<float *>(h->ipfb_y + v_bytes);
+    double *scr = reinterpret_cast<double *>(h->ipfb_scr), *v = reinterpret_cast<double *>(h->ipfb_y);
     if (plan && h->ipfb_rows < nblock) {
         SDBE_CK(h, cudaDeviceSynchronize());  // calls on other streams may still read the scratch
         SDBE_CK(h, with_taps(ntap, [&](auto nt) { return launch_factor<decltype(nt)::value>(nblock, h->ipfb_tab, scr, st); }));
