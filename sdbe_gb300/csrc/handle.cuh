@@ -63,7 +63,7 @@ struct sdbe_resampler {
     int64_t ing_hdr_bytes = 0;
     sdbe_reform_state reform{-1, -1, -1, -1, -1, 0, 0, 0};  // 8pac batches: reform state
     sdbe_reform_state *reform_dev = nullptr;                // kernel's output state
-    double *ipfb_tab = nullptr;   // inverse PFB: [2][ntap][32768] band of P P^T and P taps (FP64)
+    double *ipfb_tab = nullptr;   // inverse PFB: [3][ntap][32768] band of P P^T, P taps, taps over the middle one (FP64)
     int ipfb_ntap = 0;
     uint8_t *ipfb_y = nullptr;    // inverse PFB scratch, grown to the largest call: with a kept factor the
                                   // substituted values [nblock][32768] f64, then y [nblock][32768] f32

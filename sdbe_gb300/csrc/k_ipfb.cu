@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(128) k_ipfb_solve(const float *__restrict__ y,
 
 // fac layout: [nblock][NT][L]: entries 0..NT-2 = L[m][m-1-k], entry NT-1 = 1/d_m.
 template <int NT>
-__global__ void __launch_bounds__(128) k_ipfb_factor(int64_t nblock, const double *__restrict__ tab,
+__global__ void __launch_bounds__(128) k_ipfb_factor(int64_t nblock, double *__restrict__ tab,
                                                      double *__restrict__ fac) {
     constexpr int B = NT - 1;
     constexpr int L = kNA;
@@ -143,6 +143,11 @@ __global__ void __launch_bounds__(128) k_ipfb_factor(int64_t nblock, const doubl
     double a[NT];
 #pragma unroll
     for (int d = 0; d < NT; ++d) a[d] = tab[d * L + p];
+    // The backward sweep runs on z w_c, c the middle tap (0.5 and above, but for
+    // two taps' 0.08): scaled in the factor's 1/d, and the projection's tap c is 1.
+    const double wc = tab[(NT + NT / 2) * L + p], wci = 1.0 / wc;
+#pragma unroll
+    for (int d = 0; d < NT; ++d) tab[(2 * NT + d) * L + p] = tab[(NT + d) * L + p] * wci;
     double pl[B][B], pd[B], pdi[B];  // as in k_ipfb_solve
 #pragma unroll
     for (int k = 0; k < B; ++k) {
@@ -167,7 +172,7 @@ __global__ void __launch_bounds__(128) k_ipfb_factor(int64_t nblock, const doubl
         double *row = fac + m * NT * L + p;
 #pragma unroll
         for (int k = 0; k < B; ++k) row[k * L] = l[k];
-        row[B * L] = dinv;
+        row[B * L] = dinv * wc;
 #pragma unroll
         for (int k = B - 1; k >= 1; --k) {
             pd[k] = pd[k - 1];
@@ -228,11 +233,12 @@ __device__ __forceinline__ void copy_wait() {  // all but the last N groups have
 
 // Forward and backward substitution with a kept factor; v: [nblock][L] scratch.
 // One warp per CTA, so that 1024 warps leave no sub-partition with more than
-// two.  FP64 issue (64 cycles a warp instruction, 11 for a row of four taps) is
+// two.  FP64 issue (64 cycles a warp instruction, 10 for a row of four taps) is
 // the bound, if a row's values are there: four instructions of the forward
 // sweep are a fraction of a trip to DRAM, so kRing rows are on their way.  48
 // blocks, four taps: 60.8 us with one row ahead and 14 FP64 instructions a row,
-// now 38.0, of which two warps' instructions take 33.4.
+// 38.0 with 11 (two warps' instructions take 33.4); a tap of 1 in the
+// projection takes one more away (the call 50.1 -> 48.2 us).
 template <int NT>
 __global__ void __launch_bounds__(32) k_ipfb_apply(const float *__restrict__ y, int64_t nblock,
                                                    const double *__restrict__ tab, const double *__restrict__ fac,
@@ -245,7 +251,7 @@ __global__ void __launch_bounds__(32) k_ipfb_apply(const float *__restrict__ y, 
     const int lane = threadIdx.x, p = blockIdx.x * 32 + lane;
     double w[NT];
 #pragma unroll
-    for (int d = 0; d < NT; ++d) w[d] = tab[(NT + d) * L + p];
+    for (int d = 0; d < NT; ++d) w[d] = d == NT / 2 ? 1.0 : tab[(2 * NT + d) * L + p];
     double pw[B];
 #pragma unroll
     for (int k = 0; k < B; ++k) pw[k] = 0.0;
@@ -301,9 +307,13 @@ __global__ void __launch_bounds__(32) k_ipfb_apply(const float *__restrict__ y, 
 #pragma unroll
         for (int k = 1; k <= B; ++k) z -= nl[k - 1][k - 1] * nz[k - 1];
         // x_{m+B} = sum_t w[t] z_{m+B-t}, t = 0..B  (z_{m..m+B} known)
-        double x = w[B] * z;
+        // (w[NT / 2] is 1, and z_m itself for two taps)
+        constexpr int c = NT / 2;
+        double x = c == B ? z : nz[B - 1 - c];
 #pragma unroll
-        for (int t = 0; t < B; ++t) x += w[t] * nz[B - 1 - t];
+        for (int t = 0; t < B; ++t)
+            if (t != c) x += w[t] * nz[B - 1 - t];
+        if constexpr (c != B) x += w[B] * z;
         out[(m + B) * L + p] = rounded_f32(x);
 #pragma unroll
         for (int k = B - 1; k >= 1; --k) {
@@ -355,7 +365,7 @@ cudaError_t launch_solve(const float *y, int64_t nblock, const double *tab, doub
     return cudaGetLastError();
 }
 template <int NT>
-cudaError_t launch_factor(int64_t nblock, const double *tab, double *fac, cudaStream_t st) {
+cudaError_t launch_factor(int64_t nblock, double *tab, double *fac, cudaStream_t st) {
     k_ipfb_factor<NT><<<kNA / 128, 128, 0, st>>>(nblock, tab, fac);
     return cudaGetLastError();
 }
@@ -403,7 +413,7 @@ extern "C" int sdbe_inverse_pfb(sdbe_resampler *h, const void *spec_c64, int64_t
             h->ipfb_ntap = 0;
         }
         h->ipfb_rows = 0;
-        SDBE_CK(h, cudaMalloc(&h->ipfb_tab, tab.size() * sizeof(double)));
+        SDBE_CK(h, cudaMalloc(&h->ipfb_tab, (tab.size() + static_cast<size_t>(ntap) * kNA) * sizeof(double)));
         SDBE_CK(h, cudaMemcpyAsync(h->ipfb_tab, tab.data(), tab.size() * sizeof(double), cudaMemcpyHostToDevice, st));
         SDBE_CK(h, cudaStreamSynchronize(st));  // tab is freed on return
         h->ipfb_ntap = ntap;
