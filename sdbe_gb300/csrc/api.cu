@@ -260,6 +260,22 @@ int plan_call(sdbe_resampler *h, const void *packets, int64_t n_packets, int32_t
     return SDBE_OK;
 }
 
+// The same `bytes` of both pols in one copy where the pols' distances are
+// within the device's largest pitch of a 2D copy, else in two.  The limit
+// reads 2^31 - 1: the spectra of a handle of 2047 frames and the payloads of
+// 2048 batches are above it.  (Driver 580.159 was seen to take larger pitches;
+// the runtime's documentation says that it refuses them.)
+cudaError_t copy_pols(const sdbe_resampler *h, void *dst, int64_t dst_pitch, const void *src, int64_t src_pitch,
+                      size_t bytes, cudaMemcpyKind kind, cudaStream_t st) {
+    if (std::max(dst_pitch, src_pitch) <= h->max_pitch)
+        return cudaMemcpy2DAsync(dst, dst_pitch, src, src_pitch, bytes, 2, kind, st);
+    cudaError_t e = cudaMemcpyAsync(dst, src, bytes, kind, st);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(static_cast<uint8_t *>(dst) + dst_pitch, static_cast<const uint8_t *>(src) + src_pitch,
+                            bytes, kind, st);
+    return e;
+}
+
 // Payload packets [lo, hi) of both pols are final: send them to the host on
 // the copy stream while the next wave computes.
 int ship_call(CallPlan &c, int64_t lo, int64_t hi) {
@@ -267,9 +283,9 @@ int ship_call(CallPlan &c, int64_t lo, int64_t hi) {
     if (!c.host_out || hi <= lo) return SDBE_OK;
     SDBE_CK(h, cudaEventRecord(h->wave_ev, c.st));
     SDBE_CK(h, cudaStreamWaitEvent(h->copy_out, h->wave_ev, 0));
-    SDBE_CK(h, cudaMemcpy2DAsync(static_cast<uint8_t *>(c.out) + lo * c.pkt_stride, c.out_pol_stride,
-                                 c.dev_out + lo * c.pkt_stride, c.out_pol_stride, (hi - lo) * c.pkt_stride, 2,
-                                 cudaMemcpyDeviceToHost, h->copy_out));
+    SDBE_CK(h, copy_pols(h, static_cast<uint8_t *>(c.out) + lo * c.pkt_stride, c.out_pol_stride,
+                         c.dev_out + lo * c.pkt_stride, c.out_pol_stride, (hi - lo) * c.pkt_stride,
+                         cudaMemcpyDeviceToHost, h->copy_out));
     return SDBE_OK;
 }
 
@@ -397,9 +413,9 @@ int complete_call(CallPlan &c, sdbe_result *result) {
     const int64_t total = h->carry + c.n_frames_out * kSnapsPerFrame;
     const int64_t new_carry = total - c.n_batches * kBatchSnaps;
     if (c.n_batches > 0 && new_carry > 0) {
-        const size_t pitch = static_cast<size_t>(h->spec_pol_stride) * sizeof(uint32_t);
-        SDBE_CK(h, cudaMemcpy2DAsync(h->spec, pitch, h->spec + c.n_batches * kBatchSnaps * kGroups, pitch,
-                                     new_carry * kGroups * sizeof(uint32_t), 2, cudaMemcpyDeviceToDevice, st));
+        const int64_t pitch = h->spec_pol_stride * static_cast<int64_t>(sizeof(uint32_t));
+        SDBE_CK(h, copy_pols(h, h->spec, pitch, h->spec + c.n_batches * kBatchSnaps * kGroups, pitch,
+                             new_carry * kGroups * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st));
     }
     h->carry = new_carry;
     h->last_stream = st;
@@ -631,6 +647,10 @@ int sdbe_create(const sdbe_config *cfg, sdbe_resampler **out) {
         cudaGetLastError();
         return fail(nullptr, code, m);
     };
+    int pitch = 0;
+    if (cudaDeviceGetAttribute(&pitch, cudaDevAttrMaxPitch, cfg->device) != cudaSuccess)
+        return bail(SDBE_ERR_CUDA, "device attribute");
+    h->max_pitch = pitch;
     if (configure_fft_kernels() != cudaSuccess) return bail(SDBE_ERR_CUDA, "kernel attribute setup failed");
     if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaStreamCreateWithFlags(&h->copy_in, cudaStreamNonBlocking) != cudaSuccess ||

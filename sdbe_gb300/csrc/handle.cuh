@@ -20,6 +20,7 @@ struct sdbe_resampler {
     int64_t max_snaps = 0;
     uint32_t *spec = nullptr;     // [2][max_snaps][2048] packed spectra
     int64_t spec_pol_stride = 0;  // words
+    int64_t max_pitch = 0;        // largest pitch of a 2D copy on the device, bytes
     int32_t *counts = nullptr;    // [max_frames] per-frame packets, then [1] rejected; then, 256-byte aligned,
     uint32_t *bitmap = nullptr;   // [max_frames][64] (the same allocation)
     float *ts = nullptr;          // [2][wave*143*32768] stage-A time series
