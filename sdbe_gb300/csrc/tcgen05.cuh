@@ -125,11 +125,14 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *mbar, uint32_t parity, uint6
 }
 
 __device__ __forceinline__ bool flag_set(const int *flag) { return *reinterpret_cast<const volatile int *>(flag) != 0; }
-// mbar_wait that raises `flag` (shared memory) on time-out; once it is raised, waits return at once.
+// mbar_wait by a whole warp that raises `flag` (shared memory) on time-out; once
+// it is raised, waits return at once.  Lanes poll for themselves and may see the
+// phase complete at different times, so the warp votes (and joins again after
+// the slow way): the instructions behind a wait are often .sync.aligned.
 __device__ __forceinline__ void wait_or_flag(uint64_t *mbar, uint32_t parity, int *flag) {
-    if (mbar_poll(mbar, parity)) return;
-    if (flag_set(flag)) return;
-    if (!mbar_wait(mbar, parity)) *reinterpret_cast<volatile int *>(flag) = 1;
+    if (__all_sync(0xffffffffu, mbar_poll(mbar, parity))) return;
+    if (!flag_set(flag) && !mbar_wait(mbar, parity)) *reinterpret_cast<volatile int *>(flag) = 1;
+    __syncwarp();
 }
 __device__ __forceinline__ void fence_mbar_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
 
