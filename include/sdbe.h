@@ -454,6 +454,10 @@ int sdbe_fp32_fma_rate(int32_t device, double *tflops, double *ms);
  * the context stays usable.  The call after it returns SDBE_ERR_CUDA.  Used
  * by the tests of the failure path; limit_ns must be in [1e3, 1e9]. */
 int sdbe_test_tc_timeout(sdbe_resampler *h, int64_t limit_ns);
+/* The same for the FP32 kernels: from now on h's stage-A (stage 1) or stage-BC
+ * (stage 2) launches expect one barrier arrival that never comes; their waits
+ * run out after the usual second. */
+int sdbe_test_fft_timeout(sdbe_resampler *h, int32_t stage);
 
 /* ---- test hook: group assembly decisions (no counterpart in the reference) */
 /* Copies to host memory the accept flag (1: inserted into a group) that the

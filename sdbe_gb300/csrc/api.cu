@@ -910,6 +910,13 @@ int sdbe_profile_read(sdbe_resampler *h, sdbe_profile *out) {
     return SDBE_OK;
 }
 
+int sdbe_test_fft_timeout(sdbe_resampler *h, int32_t stage) {
+    if (!h) return SDBE_ERR_ARG;
+    if (stage < 1 || stage > 2) return fail(h, SDBE_ERR_ARG, "stage must be 1 or 2");
+    h->tw.withhold = stage;
+    return SDBE_OK;
+}
+
 int sdbe_last_error(const sdbe_resampler *h, char *buf, size_t n) {
     if (!buf || n == 0) return SDBE_ERR_ARG;
     const std::string &m = h ? h->err : thread_error();

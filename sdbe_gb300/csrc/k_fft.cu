@@ -677,7 +677,7 @@ __global__ void __launch_bounds__(kNTA, 1) k_swarm_c2r(const __grid_constant__ S
         tc5::mbar_init(&P.full[0], 1);
         tc5::mbar_init(&P.full[1], 1);
         tc5::mbar_init(&P.read, kNTA / 32);
-        tc5::mbar_init(&P.second, kNTA / 32);
+        tc5::mbar_init(&P.second, kNTA / 32 + (tw.withhold == 1 ? 1 : 0));
         tc5::fence_mbar_init();
         P.err = 0;
         // the first spectra on their way while the tables load
@@ -702,13 +702,16 @@ __global__ void __launch_bounds__(kNTA, 1) k_swarm_c2r(const __grid_constant__ S
     __syncthreads();  // the four warps of a quarter read one table
     tc5::fence_after();
     const LastTw lt = last_tw(T);  // once per CTA
-    auto wait = [&](uint64_t *bar, uint32_t parity) { tc5::wait_or_flag(bar, parity, &P.err); };
+    auto wait = [&](uint64_t *bar, uint32_t parity) { return tc5::wait_or_flag(bar, parity, &P.err); };
+    // The first item whose spectrum this thread did not see land (after a
+    // wait has run out); none is asked for after that.
+    uint32_t lost = ~0u;
     // Input columns of the k-th item (its spectrum in buffer k & 1), DFT-32,
     // parked.  The first pass takes Z[col + 512 r] from the packed bins X[k]
     // (k < 16384; the Nyquist bin X[16384] = 0, Im X[0] dropped), each
     // Hermitian pair once with its mirror half from lane ^ 16.
     auto input = [&](uint32_t k) {
-        wait(&P.full[k & 1], k >> 1);
+        if (!wait(&P.full[k & 1], k >> 1) && lost == ~0u) lost = k;
         const uint32_t *cur = sp + (k & 1) * kGroups;
         float2 v[32], w[16];
         for_r(std::make_integer_sequence<int, 16>{}, [&](auto pc) { w[decltype(pc)::value] = c2r_tw<decltype(pc)::value>(wc); });
@@ -749,8 +752,9 @@ __global__ void __launch_bounds__(kNTA, 1) k_swarm_c2r(const __grid_constant__ S
         if (item + G < n_items) input(k + 1);
         wait(&P.second, k);
         // every warp is done with this item's spectrum (its input columns
-        // came before its second pass): the buffer takes the item after next
-        if (threadIdx.x == 0 && item + 2 * G < n_items) fetch(item + 2 * G, k & 1);
+        // came before its second pass): the buffer takes the item after next,
+        // unless a copy's wait ran out
+        if (threadIdx.x == 0 && item + 2 * G < n_items && lost == ~0u) fetch(item + 2 * G, k & 1);
         const SegA &g = S.s[seg_of(S, item)];
         const int64_t local = item - g.item0;
         const int64_t pol = local >= g.n_snaps, s = local - pol * g.n_snaps;
@@ -769,6 +773,12 @@ __global__ void __launch_bounds__(kNTA, 1) k_swarm_c2r(const __grid_constant__ S
         first = spare;
         spare = second;
         second = t;
+    }
+    // no copy outlives the CTA: one more bounded wait for the lost item's, and
+    // for item 1's, asked for together with item 0's
+    if (threadIdx.x == 0 && lost != ~0u) {
+        tc5::mbar_wait(&P.full[lost & 1], lost >> 1);
+        if (lost == 0 && blockIdx.x + G < n_items) tc5::mbar_wait(&P.full[1], 0);
     }
     tc5::fence_before();
     __syncthreads();
@@ -837,7 +847,7 @@ __global__ void __launch_bounds__(kNTB, 1) k_resample(const __grid_constant__ Se
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (tid == 0) {
         uint64_t *bars[6] = {&P.xfree, &P.pass2, &P.pass3, &P.pass4, &P.taken, &P.inv2};
-        for (uint64_t *b : bars) tc5::mbar_init(b, kNTB / 32);
+        for (uint64_t *b : bars) tc5::mbar_init(b, kNTB / 32 + (b == &P.pass2 && tw.withhold == 2 ? 1 : 0));
         tc5::fence_mbar_init();
         P.err = 0;
     }

@@ -129,10 +129,13 @@ __device__ __forceinline__ bool flag_set(const int *flag) { return *reinterpret_
 // it is raised, waits return at once.  Lanes poll for themselves and may see the
 // phase complete at different times, so the warp votes (and joins again after
 // the slow way): the instructions behind a wait are often .sync.aligned.
-__device__ __forceinline__ void wait_or_flag(uint64_t *mbar, uint32_t parity, int *flag) {
-    if (__all_sync(0xffffffffu, mbar_poll(mbar, parity))) return;
-    if (!flag_set(flag) && !mbar_wait(mbar, parity)) *reinterpret_cast<volatile int *>(flag) = 1;
+// Returns whether this lane saw the phase complete.
+__device__ __forceinline__ bool wait_or_flag(uint64_t *mbar, uint32_t parity, int *flag) {
+    if (__all_sync(0xffffffffu, mbar_poll(mbar, parity))) return true;
+    const bool done = !flag_set(flag) && mbar_wait(mbar, parity);
+    if (!done) *reinterpret_cast<volatile int *>(flag) = 1;
     __syncwarp();
+    return done;
 }
 __device__ __forceinline__ void fence_mbar_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
 
