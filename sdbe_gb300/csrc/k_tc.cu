@@ -452,7 +452,12 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_fft(const __grid_constant_
             for (int k = 0; k < G::NPIN; ++k) bulk_copy(aop + k * STAGE, a.f1 + k * STAGE1, STAGE1, &full[0]);
             issue_stream(0);
             issue_stream(1);
-            if (!mbar_wait(&full[0], 0)) err = true;
+            pend |= 1u;
+            pend_g[0] = 0;
+            if (mbar_wait(&full[0], 0))
+                pend &= ~1u;
+            else
+                err = true;
         } else {
             for (int i = 0; i < NRING - 1; ++i) issue_copy(i);
         }
