@@ -292,7 +292,8 @@ int sdbe_process_multi(sdbe_resampler *const *handles, const sdbe_stream_desc *d
                        void *stream, sdbe_result *results);
 
 /* Wait for all work the handle issued (its streams and the last stream passed
- * to sdbe_process). */
+ * to sdbe_process).  SDBE_ERR_CUDA if a kernel of that work gave up on a
+ * barrier wait and no call has returned that error yet. */
 int sdbe_sync(sdbe_resampler *h);
 int sdbe_get_state(sdbe_resampler *h, sdbe_state *st);
 int sdbe_set_state(sdbe_resampler *h, const sdbe_state *st);
@@ -451,8 +452,8 @@ int sdbe_fp32_fma_rate(int32_t device, double *tflops, double *ms);
  * mbarrier wait of that launch by limit_ns nanoseconds.  The wait that
  * depends on the withheld signal runs out; the kernel records the time-out
  * in h's status flag, stops waiting, frees its tensor memory and returns, so
- * the context stays usable.  The call after it returns SDBE_ERR_CUDA.  Used
- * by the tests of the failure path; limit_ns must be in [1e3, 1e9]. */
+ * the context stays usable.  A call that synchronizes, and every later one,
+ * returns SDBE_ERR_CUDA.  Used by the tests of the failure path; limit_ns must be in [1e3, 1e9]. */
 int sdbe_test_tc_timeout(sdbe_resampler *h, int64_t limit_ns);
 /* The same for the FP32 kernels: from now on h's stage-A (stage 1) or stage-BC
  * (stage 2) launches expect one barrier arrival that never comes; their waits

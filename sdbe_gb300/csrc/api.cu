@@ -31,6 +31,7 @@ int fail(sdbe_resampler *h, int code, const std::string &msg) {
 
 int check_status(sdbe_resampler *h) {
     if (!*reinterpret_cast<volatile int *>(h->tc_status_host)) return SDBE_OK;
+    h->timeout_told = true;
     return fail(h, SDBE_ERR_CUDA, "a transform timed out on its mbarrier wait");
 }
 
@@ -424,6 +425,7 @@ int complete_call(CallPlan &c, sdbe_result *result) {
     if (need_sync) {
         SDBE_CK(h, cudaStreamSynchronize(st));
         if (c.host_out) SDBE_CK(h, cudaStreamSynchronize(h->copy_out));
+        if (int rc = check_status(h)) return rc;
     }
     if (result) {
         std::vector<int32_t> cnt(static_cast<size_t>(h->cfg.max_frames) + 1);
@@ -816,7 +818,7 @@ int sdbe_sync(sdbe_resampler *h) {
     if (h->last_stream) SDBE_CK(h, cudaStreamSynchronize(h->last_stream));
     SDBE_CK(h, cudaStreamSynchronize(h->stream));
     SDBE_CK(h, cudaStreamSynchronize(h->copy_out));
-    return SDBE_OK;
+    return h->timeout_told ? SDBE_OK : check_status(h);
 }
 
 int sdbe_get_state(sdbe_resampler *h, sdbe_state *st) {
@@ -994,8 +996,8 @@ int sdbe_swarm_c2r(sdbe_resampler *h, const uint32_t *spec, int64_t n_snapshots,
     if (!h || n_snapshots < 0 || (n_snapshots > 0 && (!spec || !out))) return fail(h, SDBE_ERR_ARG, "bad argument");
     if (unaligned(spec, 16) || unaligned(out, 16)) return fail(h, SDBE_ERR_ARG, "spectra and output must be 16-byte aligned");
     DeviceGuard g(h->cfg.device);
-    if (h->cfg.precision != SDBE_PRECISION_FP32) return tc_swarm_c2r(h, spec, n_snapshots, out, pick(h, stream));
     if (int rc = check_status(h)) return rc;
+    if (h->cfg.precision != SDBE_PRECISION_FP32) return tc_swarm_c2r(h, spec, n_snapshots, out, pick(h, stream));
     SDBE_CK(h, launch_swarm_c2r(spec, 0, 0, n_snapshots, 1, out, 0, h->tw, pick(h, stream)));
     return SDBE_OK;
 }
@@ -1022,6 +1024,7 @@ int sdbe_resample_chunks(sdbe_resampler *h, const float *in, int64_t n_chunks, f
     if (!h || n_chunks < 0 || (n_chunks > 0 && (!in || !out))) return fail(h, SDBE_ERR_ARG, "bad argument");
     if (unaligned(in, 16) || unaligned(out, 16)) return fail(h, SDBE_ERR_ARG, "input and output must be 16-byte aligned");
     DeviceGuard g(h->cfg.device);
+    if (int rc = check_status(h)) return rc;
     if (h->cfg.precision != SDBE_PRECISION_FP32) return tc_resample_chunks(h, in, n_chunks, out, pick(h, stream));
     ResampleOut o{};
     o.fout = out;

@@ -139,6 +139,7 @@ int finish(sdbe_resampler *h, void *out, uint8_t *dev_out, int64_t n_ships, uint
     if ((flags & SDBE_OUT_HOST) && n_ships > 0)
         SDBE_CK(h, cudaMemcpyAsync(out, dev_out, n_ships * group_bytes(flags), cudaMemcpyDeviceToHost, st));
     SDBE_CK(h, cudaStreamSynchronize(st));
+    if (int rc = check_status(h)) return rc;
     h->last_stream = st;
     if (n_groups) *n_groups = static_cast<int32_t>(n_ships);
     return SDBE_OK;

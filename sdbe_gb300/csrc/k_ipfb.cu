@@ -403,6 +403,7 @@ extern "C" int sdbe_inverse_pfb(sdbe_resampler *h, const void *spec_c64, int64_t
     if (nblock > (int64_t(1) << 20)) return fail(h, SDBE_ERR_CAPACITY, "at most 2^20 blocks per call");
     DeviceGuard g(h->cfg.device);
     if (!g.ok) return fail(h, SDBE_ERR_CUDA, "cudaSetDevice failed");
+    if (int rc = check_status(h)) return rc;
     cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : h->stream;
     if (h->ipfb_ntap != ntap) {
         const std::vector<double> tab = ipfb_table(ntap);

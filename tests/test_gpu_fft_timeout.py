@@ -49,6 +49,53 @@ def test_hook_refuses_bad_arguments(N):
 
 
 @pytest.mark.parametrize("stage", [1, 2])
+def test_calls_that_wait_report_it(N, stream, stage):
+    """A call that synchronizes reports its own time-out, as does sdbe_sync."""
+    import torch
+
+    from sdbe_gb300 import Resampler
+
+    p, b0, _ = stream
+    for host in (True, False):
+        with Resampler(trim_mhz=150, max_frames=2) as rs:
+            N.check(N.lib().sdbe_test_fft_timeout(rs.handle, stage), rs.handle)
+            if host:
+                _timed_out(N, lambda: rs.process(p[:4096], 2, b0))
+            else:
+                out = torch.empty(rs.output_bytes(2), dtype=torch.uint8, device="cuda")
+                rs.process(torch.from_numpy(p[:4096]).cuda(), 2, b0, out=out, want_result=False)
+                _timed_out(N, rs.sync)
+
+
+@pytest.mark.parametrize("stage,name", [(1, "sdbe_swarm_c2r"), (2, "sdbe_resample_chunks")])
+def test_stage_functions_report_it(N, stage, name):
+    import torch
+
+    from sdbe_gb300 import Resampler
+
+    a, b = (torch.zeros(36608, device="cuda") for _ in range(2))
+    with Resampler(max_frames=2) as rs:
+        N.check(N.lib().sdbe_test_fft_timeout(rs.handle, stage), rs.handle)
+        fn = getattr(N.lib(), name)
+        assert fn(rs.handle, a.data_ptr(), 1, b.data_ptr(), None) == N.OK
+        _timed_out(N, rs.sync)
+        assert fn(rs.handle, a.data_ptr(), 1, b.data_ptr(), None) == N.ERR_CUDA
+
+
+@pytest.mark.parametrize("stage", [1, 2])
+def test_ingest_reports_it(N, stage):
+    from sdbe_gb300 import Resampler, synth
+
+    spec = synth.config1()
+    spec.n_frames = 4
+    p = synth.generate(spec)
+    with Resampler(max_frames=143) as rs:
+        rs.ingest(p)
+        N.check(N.lib().sdbe_test_fft_timeout(rs.handle, stage), rs.handle)
+        _timed_out(N, rs.ingest_flush)
+
+
+@pytest.mark.parametrize("stage", [1, 2])
 def test_wait_that_runs_out(N, stream, stage):
     """Launches of several items per CTA and of one; then a fresh handle."""
     from sdbe_gb300 import Resampler
