@@ -510,6 +510,7 @@ int fft_chain_multi(std::vector<CallPlan> &cs) {
             A.s[A.n] = SegA{h->spec, h->ts, h->spec_pol_stride, 0, kBatchSnaps, h->ts_pol_stride, A.n_items};
             A.n_items += 2 * kBatchSnaps;
             ++A.n;
+            A.status.add(h->tc_status);
             ResampleOut o{};
             o.fout = h->fout;
             o.fout_pol_stride = static_cast<int64_t>(kChunks) * kNC;
@@ -520,6 +521,7 @@ int fft_chain_multi(std::vector<CallPlan> &cs) {
             first.push_back(i);
         }
         if (!first.empty()) {
+            B.status = A.status;
             SDBE_CK(h0, launch_swarm_c2r_segs(A, h0->tw, st));
             SDBE_CK(h0, launch_resample_segs(1, B, h0->tw, st));
             h0->launches += 2;
@@ -560,6 +562,7 @@ int fft_chain_multi(std::vector<CallPlan> &cs) {
                             A.n_items};
             A.n_items += 2 * nb * kBatchSnaps;
             ++A.n;
+            A.status.add(h->tc_status);
             const PayloadTarget &t = cs[i].pt;
             ResampleOut o{};
             o.out = t.base;
@@ -575,6 +578,7 @@ int fft_chain_multi(std::vector<CallPlan> &cs) {
             act.emplace_back(i, nb);
         }
         if (act.empty()) break;
+        B.status = A.status;
         size_t slot;
         SDBE_CK(h0, timed_begin(h0, 0, A.n_items, st, &slot));
         SDBE_CK(h0, launch_swarm_c2r_segs(A, h0->tw, st));
@@ -770,9 +774,12 @@ int sdbe_process_multi(sdbe_resampler *const *hs, const sdbe_stream_desc *d, int
     const int chain_rc = fft_chain_multi(c);
     for (auto &ci : c) ci.h->shipping = false;
     if (chain_rc) return chain_rc;
-    for (int i = 0; i < n; ++i)
-        if (int rc = complete_call(c[i], results ? results + i : nullptr)) return rc;
-    return SDBE_OK;
+    int first_rc = SDBE_OK;  // one stream's time-out leaves the others' state advanced
+    for (int i = 0; i < n; ++i) {
+        const int rc = complete_call(c[i], results ? results + i : nullptr);
+        if (!first_rc) first_rc = rc;
+    }
+    return first_rc;
 }
 
 int sdbe_header_template(int32_t t0_sec, int32_t t0_clk, uint32_t ref_epoch, sdbe_time_template *out) {

@@ -248,6 +248,7 @@ struct TcfASeg {
     int64_t spec_pol_stride, snap0, n_snaps;
     void *out;               // float, or FP16 x 2^-2
     int64_t out_pol_stride;  // elements
+    int *status;             // the handle's status flag
 };
 int tcf_prepare(sdbe_resampler *h, cudaStream_t st);
 int tcf_stage_a(sdbe_resampler *h, const TcfASeg *segs, int n_segs, int n_pols, bool half_out, cudaStream_t st);
@@ -264,6 +265,7 @@ struct TcfBCSeg {
     int64_t n_chunks;
     int skip;
     ResampleOut o;
+    int *status;             // the handle's status flag
 };
 int tcf_stage_bc(sdbe_resampler *h, const TcfBCSeg *segs, int n_segs, int n_pols, int mode, cudaStream_t st);
 cudaError_t tcf_to_half(const float *in, void *out, int64_t n_floats, cudaStream_t st);

@@ -783,7 +783,7 @@ __global__ void __launch_bounds__(kNTA, 1) k_swarm_c2r(const __grid_constant__ S
     tc5::fence_before();
     __syncthreads();
     if (warp == 0) tc5::tmem_free(P.tmem, kColsA);
-    if (threadIdx.x == 0 && tc5::flag_set(&P.err)) *reinterpret_cast<volatile int *>(tw.status) = 1;
+    if (threadIdx.x == 0 && tc5::flag_set(&P.err)) S.status.raise();
 }
 
 // ---------------------------------------------------------------------------
@@ -1134,7 +1134,7 @@ __global__ void __launch_bounds__(kNTB, 1) k_resample(const __grid_constant__ Se
     tc5::fence_before();
     __syncthreads();
     if (warp == 0) tc5::tmem_free(P.tmem, kColsB);
-    if (tid == 0 && tc5::flag_set(&P.err)) *reinterpret_cast<volatile int *>(tw.status) = 1;
+    if (tid == 0 && tc5::flag_set(&P.err)) S.status.raise();
 }
 
 // SwarmR2C alone: complex64 [n][18305] spectra (persistent over chunks).
@@ -1504,6 +1504,7 @@ cudaError_t launch_swarm_c2r(const uint32_t *spec, int64_t spec_pol_stride, int6
     S.n = 1;
     S.n_items = n_snaps * n_pols;
     S.s[0] = SegA{spec, out, spec_pol_stride, snap0, n_snaps, out_pol_stride, 0};
+    S.status.add(tw.status);
     return launch_swarm_c2r_segs(S, tw, st);
 }
 
@@ -1514,6 +1515,7 @@ cudaError_t launch_resample(int mode, const float *in, int64_t in_pol_stride, in
     S.n = 1;
     S.n_items = n_chunks * n_pols;
     S.s[0] = SegB{in, in_pol_stride, 0, static_cast<int>(n_chunks), skip, o};
+    S.status.add(tw.status);
     return launch_resample_segs(mode, S, tw, st);
 }
 

@@ -158,7 +158,7 @@ struct TcFftArgs {
     const uint8_t *f1;                 // DFT-128 tiles [8 K-steps][4 comps][4 KB]
     const uint8_t *f2;                 // DFT-N2 tiles [K-steps][4 comps][NP rows x 16 k]
     const float2 *tw;                  // e^{-2 pi i e / (128 N2)}, e < 128 N2
-    int *status;                       // set to 1 on a barrier time-out (host-mapped)
+    StatusFlags status;                // raised on a barrier time-out
 };
 
 __device__ __forceinline__ const TcSeg &seg_of(const TcFftArgs &a, int64_t item) {
@@ -593,7 +593,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_fft(const __grid_constant_
     }
     if (OVL && y_prev && !s_err) store_out(y_prev, inv_prev);
     if (s_err && tid == 0) {  // a wait timed out: record it, let copies and MMAs in flight finish (bounded)
-        *reinterpret_cast<volatile int *>(a.status) = 1;
+        a.status.raise();
         for (int b = 0; b < NRING; ++b)
             if (pend & (1u << b)) mbar_wait(&full[b], (G::PIN ? pend_g[b] >> 1 : pend_g[b] / NRING) & 1u);
         mma_commit(&done);
@@ -758,7 +758,7 @@ static TcFftArgs one_seg(const TcSeg &g, const uint8_t *f1, const uint8_t *f2, c
     a.f1 = f1;
     a.f2 = f2;
     a.tw = tw;
-    a.status = status;
+    a.status.add(status);
     return a;
 }
 
@@ -806,7 +806,7 @@ int tc_wave_multi(const std::vector<TcWaveItem> &w, bool first, cudaStream_t st)
         x->f1 = f128;
         x->f2 = x == &B ? f143 : f128;
         x->tw = x == &B ? tw.w18304 : tw.w16384;
-        x->status = h0->tc_status;
+        for (const auto &it : w) x->status.add(it.h->tc_status);
     }
     int64_t units_a = 0, units_bc = 0;
     for (const auto &it : w) {
@@ -904,7 +904,7 @@ int tc_swarm_c2r(sdbe_resampler *h, const uint32_t *spec, int64_t n_snaps, float
     if (int rc = tc_prepare(h, st)) return rc;
     const uint8_t *f128 = static_cast<const uint8_t *>(h->tc_f128);
     if (tc_splits(h) == 2) {  // SDBE_PRECISION_TC16_FAST: straight from the packed spectra (k_tcf.cu)
-        const TcfASeg seg{spec, 0, 0, n_snaps, out, 0};
+        const TcfASeg seg{spec, 0, 0, n_snaps, out, 0, h->tc_status};
         return tcf_stage_a(h, &seg, 1, 1, false, st);
     }
     const int64_t cap = 2 * static_cast<int64_t>(h->wave) * kBatchSnaps;
@@ -940,6 +940,7 @@ int tc_resample_chunks(sdbe_resampler *h, const float *in, int64_t n_chunks, flo
             b.bins = h->tcf_bins;
             b.n_chunks = n;
             b.skip = h->skip;
+            b.status = h->tc_status;
             b.o.fout = out + c0 * kNC;
             if (int rc = tcf_stage_bc(h, &b, 1, 1, 5, st)) return rc;
         }

@@ -346,7 +346,7 @@ struct ArgsInv {
     SegInv s[kMaxSegs];
     const uint8_t *g;        // inverse DFT-32 then DFT-16 matrices, pre-tiled
     const float2 *tab;       // the kInvTabLen twiddle values
-    int *status;             // set to 1 on a barrier time-out (host-mapped)
+    StatusFlags status;      // raised on a barrier time-out
     uint64_t wait_ns;        // bound of every mbarrier wait
     int withhold;            // 1: team 0 withholds its first stage commit (test of the time-out path)
 };
@@ -1019,7 +1019,7 @@ __device__ __forceinline__ void inv_phase(const ArgsInv &a, const Sched sc, uint
     fence_before();
     __syncthreads();
     if (threadIdx.x == 0 && *reinterpret_cast<const volatile int *>(&ctl.err) != 0)
-        *reinterpret_cast<volatile int *>(a.status) = 1;
+        a.status.raise();
 }
 
 template <int IN, int OUT>
@@ -1065,7 +1065,7 @@ struct ArgsFwd {
     SegFwd s[kMaxSegs];
     const uint8_t *g;        // forward DFT-16, DFT-8, DFT-11, DFT-13 matrices, pre-tiled
     const float2 *tab;       // the kFwdTabLen twiddle values
-    int *status;
+    StatusFlags status;
     uint64_t wait_ns;        // bound of every mbarrier wait
 };
 
@@ -1437,7 +1437,7 @@ __device__ __forceinline__ void fwd_phase(const ArgsFwd &a, const Sched sc, uint
     }
     fence_before();
     __syncthreads();
-    if (threadIdx.x == 0 && err_set(ctl)) *reinterpret_cast<volatile int *>(a.status) = 1;
+    if (threadIdx.x == 0 && err_set(ctl)) a.status.raise();
 }
 
 __global__ void __launch_bounds__(kThreads, 1) k_tcf_fwd(const __grid_constant__ ArgsFwd a) {
@@ -1662,7 +1662,7 @@ void build_a(sdbe_resampler *h, const TcfASeg *segs, int n_segs, int n_pols, Arg
     }
     A.g = blob_of(h);
     A.tab = reinterpret_cast<const float2 *>(blob_of(h) + kBlobInvTab);
-    A.status = h->tc_status;
+    for (int i = 0; i < n_segs; ++i) A.status.add(segs[i].status);
     A.wait_ns = kWaitNs;
 }
 }  // namespace
@@ -1704,11 +1704,11 @@ void build_bc(sdbe_resampler *h, const TcfBCSeg *segs, int n_segs, int n_pols, A
     }
     B.g = blob_of(h) + kBlobFwdG;
     B.tab = reinterpret_cast<const float2 *>(blob_of(h) + kBlobFwdTab);
-    B.status = h->tc_status;
+    for (int i = 0; i < n_segs; ++i) B.status.add(segs[i].status);
     B.wait_ns = kWaitNs;
     C.g = blob_of(h);
     C.tab = reinterpret_cast<const float2 *>(blob_of(h) + kBlobInvTab);
-    C.status = h->tc_status;
+    C.status = B.status;
     C.wait_ns = kWaitNs;
 }
 }  // namespace
@@ -1760,7 +1760,7 @@ int tcf_wave_multi(const std::vector<TcWaveItem> &w, bool first, cudaStream_t st
                           2 * per_pol * kTcfBinsLen * 4, "the tensor-core bins"))
             return rc;
         const int64_t snaps = it.nb * kBatchSnaps, chunks = it.nb * kChunks;
-        sa.push_back(TcfASeg{it.spec, it.spec_pol_stride, it.b0 * kBatchSnaps, snaps, h->ts, h->ts_pol_stride});
+        sa.push_back(TcfASeg{it.spec, it.spec_pol_stride, it.b0 * kBatchSnaps, snaps, h->ts, h->ts_pol_stride, h->tc_status});
         TcfBCSeg b{};
         b.ts = h->ts;  // FP16 in the float scratch: same element stride, half the bytes
         b.ts_pol_stride = h->ts_pol_stride;
@@ -1768,6 +1768,7 @@ int tcf_wave_multi(const std::vector<TcWaveItem> &w, bool first, cudaStream_t st
         b.bins_pol_stride = per_pol * kTcfBinsLen;
         b.n_chunks = chunks;
         b.skip = h->skip;
+        b.status = h->tc_status;
         const bool win = h->cfg.threshold_mode == SDBE_THRESH_WINDOW;
         if (first) {
             b.o.fout = h->fout;

@@ -18,6 +18,16 @@ struct ResampleOut {
 // one comparison), pol-major, starting at global item item0.
 // Passed by value as a __grid_constant__ kernel parameter.
 constexpr int kMaxSegs = 32;
+// The status flags (host-mapped) of the handles whose work a launch does: a
+// kernel whose barrier wait runs out raises all of them.
+struct StatusFlags {
+    int n;
+    int *p[kMaxSegs];
+    void add(int *flag) { p[n++] = flag; }
+    __device__ __forceinline__ void raise() const {
+        for (int i = 0; i < n; ++i) *reinterpret_cast<volatile int *>(p[i]) = 1;
+    }
+};
 struct SegA {  // stage A: snapshots snap0 .. snap0+n_snaps of each pol
     const uint32_t *spec;
     float *out;
@@ -27,6 +37,7 @@ struct SegsA {
     int64_t n_items;
     int n;
     SegA s[kMaxSegs];
+    StatusFlags status;
 };
 struct SegB {  // stage BC: n_chunks 36608-sample chunks of each pol
     const float *in;
@@ -38,6 +49,7 @@ struct SegsB {
     int64_t n_items;
     int n;
     SegB s[kMaxSegs];
+    StatusFlags status;
 };
 cudaError_t launch_swarm_c2r_segs(const SegsA &, const Twiddles &, cudaStream_t);
 cudaError_t launch_resample_segs(int mode, const SegsB &, const Twiddles &, cudaStream_t);

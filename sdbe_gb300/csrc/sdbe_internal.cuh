@@ -66,7 +66,7 @@ struct Twiddles {
     const float2 *w18304;  // exp(-2 pi i k / 18304), k < 18304
     const float2 *w32768;  // exp(-2 pi i k / 32768), k < 16384
     const float2 *w36608;  // exp(-2 pi i k / 36608), k <= 18304
-    int *status;           // set to 1 by a kernel whose barrier wait timed out (host-mapped)
+    int *status;           // the handle's status flag (host-mapped), see StatusFlags
     int withhold;          // test hook: 1 / 2, one arrival of stage A / BC never comes
 };
 

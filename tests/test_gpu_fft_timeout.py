@@ -95,6 +95,41 @@ def test_ingest_reports_it(N, stage):
         _timed_out(N, rs.ingest_flush)
 
 
+@pytest.mark.parametrize("waits", [False, True])
+@pytest.mark.parametrize("precision", ["FP32-1", "FP32-2", "TC16_FAST"])
+def test_every_handle_of_a_shared_launch_reports_it(N, stream, precision, waits):
+    """The first handle's launches time out; one handle has no batch in them."""
+    import torch
+
+    from sdbe_gb300 import Resampler
+    from sdbe_gb300.resampler import process_multi
+
+    p, b0, _ = stream
+    name, _, stage = precision.partition("-")
+    rs = [Resampler(max_frames=2, precision=getattr(N, "PRECISION_" + name)) for _ in range(4)]
+    if stage:
+        N.check(N.lib().sdbe_test_fft_timeout(rs[0].handle, int(stage)), rs[0].handle)
+    else:
+        N.check(N.lib().sdbe_test_tc_timeout(rs[0].handle, 2_000_000), rs[0].handle)
+    d = torch.from_numpy(p[:4096]).cuda()
+    outs = [torch.empty(r.output_bytes(2), dtype=torch.uint8, device="cuda") for r in rs]
+    torch.cuda.synchronize()
+    items = [(d, 2 if i != 1 else 1, b0, outs[i]) for i in range(3)]  # one frame: no batch
+    if waits:
+        _timed_out(N, lambda: process_multi(rs[:3], items, want_results=True))
+        for i in (0, 2):
+            _timed_out(N, lambda: rs[i].process(d, 1, b0, out=outs[i]))
+    else:
+        process_multi(rs[:3], items)
+        for i in (0, 2):
+            _timed_out(N, rs[i].sync)
+    for i in (1, 3):
+        rs[i].sync()
+    assert rs[1].get_state().carry_snapshots == 128
+    for r in rs:
+        r.close()
+
+
 @pytest.mark.parametrize("stage", [1, 2])
 def test_wait_that_runs_out(N, stream, stage):
     """Launches of several items per CTA and of one; then a fresh handle."""
