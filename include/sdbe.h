@@ -384,8 +384,9 @@ int sdbe_resample_chunks(sdbe_resampler *h, const float *in, int64_t n_chunks, f
 /* summary_stats + transform_reduce (.cu:66-137,953-977) in FP64:
  * out[0] = mean (quantizeOffset), out[1] = sqrt(M2/(n-1)) (quantizeThreshold).
  * The sums are of the samples minus the first one, so a large common offset
- * does not cancel digits of the variance.  Allocates n/256 (at most 1216)
- * pairs of FP64 partial sums on the stream and waits for it. */
+ * does not cancel digits of the variance.  Uses scratch of the calling thread
+ * (at most 304 pairs of FP64 partial sums and the shift) and waits for the
+ * stream. */
 int sdbe_summary_stats(const float *in, int64_t n, double *out_host, void *stream);
 
 /* Allocation-free variant of sdbe_summary_stats.  No counterpart in the

@@ -353,11 +353,15 @@ __device__ __forceinline__ void block_sum2(double &a, double &b, double *scratch
 // FP32 values (Knuth's two-sum; a square is its rounded value plus the exact
 // fma remainder), handed on in FP64: FP64 instructions, conversions included,
 // run at 1/64 of the FP32 rate, and seven of them for two samples took 28k of
-// a first-batch chunk's 65k cycles.  Two levels for the sum and three for the
-// squares leave the variance of a batch with the same error as FP64 sums
-// (1e-16 relative against exact sums; two levels for the squares: 5e-15).
+// a first-batch chunk's 65k cycles.  Three levels each (72 bits) leave
+// every sum of up to 1024 samples nearer to the exact one than FP64 sums do:
+// emulated over constants, uniform, Gaussian (offset by 1000 spreads too) and
+// log-normal samples, 64 to 1024 of them, no error in FP64's last place against
+// 5e-15 for FP64 sums.  Two levels for the sum, the form before, were off by
+// 5e-14 (64 log-normal samples) to 1.5e-12 (1024).  Past some thousand samples
+// the last level's own rounding shows (a constant's squares: 1e-13 at 14,000).
 struct Moments2 {
-    float s = 0.f, se = 0.f, q = 0.f, qe = 0.f, qf = 0.f;
+    float s = 0.f, se = 0.f, sf = 0.f, q = 0.f, qe = 0.f, qf = 0.f;
     static __device__ __forceinline__ float two_sum(float &a, float x) {  // a += x, returns the rounding error
         const float t = __fadd_rn(a, x), z = __fsub_rn(t, a);
         const float e = __fadd_rn(__fsub_rn(a, __fsub_rn(t, z)), __fsub_rn(x, z));
@@ -365,13 +369,15 @@ struct Moments2 {
         return e;
     }
     __device__ __forceinline__ void add(float x) {
-        se = __fadd_rn(se, two_sum(s, x));
+        sf = __fadd_rn(sf, two_sum(se, two_sum(s, x)));
         const float p = __fmul_rn(x, x);
         const float e = two_sum(q, p);
         qf = __fadd_rn(qf, two_sum(qe, e));
         qf = __fadd_rn(qf, two_sum(qe, __fmaf_rn(x, x, -p)));
     }
-    __device__ __forceinline__ double sum() const { return static_cast<double>(s) + static_cast<double>(se); }
+    __device__ __forceinline__ double sum() const {
+        return static_cast<double>(s) + (static_cast<double>(se) + static_cast<double>(sf));
+    }
     __device__ __forceinline__ double squares() const {
         return static_cast<double>(q) + (static_cast<double>(qe) + static_cast<double>(qf));
     }
@@ -380,13 +386,18 @@ struct Moments2 {
 // The same of samples less c.  x - c is its rounded value dh plus the exact
 // remainder dl, and (dh + dl)^2 = dh^2 + 2 dh dl + dl^2 with the products'
 // remainders.  Samples whose squares would leave FP32's range one way or the
-// other (and infinities and NaN) go to FP64 sums directly.  Over Gaussian
-// samples of six means and spreads the mean and the standard deviation are as
-// near to exact sums as with FP64 throughout.
+// other (and infinities and NaN) go to FP64 sums directly; flush() moves the
+// FP32 sums there, which a thread does every 1024 samples.
 struct Shifted2 {
     Moments2 m;
     double fs = 0.0, fq = 0.0;
     bool wide = false;  // fs and fq hold something
+    __device__ __forceinline__ void flush() {
+        fs += m.sum();
+        fq += m.squares();
+        m = Moments2{};
+        wide = true;
+    }
     __device__ __forceinline__ void add(float x, float c) {
         const float dh0 = __fsub_rn(x, c);
         if (!(fabsf(dh0) < 1e12f) || (fabsf(dh0) < 1e-10f && dh0 != 0.f)) {
@@ -398,7 +409,8 @@ struct Shifted2 {
         }
         float dh = x;
         const float dl = Moments2::two_sum(dh, -c);
-        m.se = __fadd_rn(m.se, __fadd_rn(Moments2::two_sum(m.s, dh), dl));
+        const float g = Moments2::two_sum(m.se, Moments2::two_sum(m.s, dh));
+        m.sf = __fadd_rn(m.sf, __fadd_rn(g, Moments2::two_sum(m.se, dl)));
         const float p = __fmul_rn(dh, dh), cr = __fmul_rn(2.f * dh, dl);
         const float e = Moments2::two_sum(m.q, p);
         float f = __fadd_rn(Moments2::two_sum(m.qe, e), Moments2::two_sum(m.qe, __fmaf_rn(dh, dh, -p)));
@@ -436,7 +448,7 @@ struct Sum3 {
 // valid in warp 0.  scratch: 6 * 16 floats.
 template <int NW>
 __device__ __forceinline__ void block_moments(const Moments2 &m, double &s1, double &s2, float *scratch) {
-    Sum3 s{m.s, m.se, 0.f}, q{m.q, m.qe, m.qf};
+    Sum3 s{m.s, m.se, m.sf}, q{m.q, m.qe, m.qf};
     s.merge_lanes<32>();
     q.merge_lanes<32>();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;

@@ -1374,7 +1374,7 @@ __global__ void k_quantize_flat(const float *__restrict__ in, uint32_t *__restri
 // shifted by the first one (x - in[0]): a large common offset then cancels
 // before the sums, not in the variance (the shifted-data algorithm; the
 // finalizers add in[0] back to the mean).  A thread's sums are unevaluated
-// FP32 ones (Shifted2): with four FP64 instructions a sample the kernel took
+// FP32 ones (Shifted2; FP64 every 1024 samples): with four FP64 instructions a sample the kernel took
 // 27 us for 2^22 samples that 3 us would read.  A batch of 1.1 million samples
 // is 14 a thread: all loaded at once, and the block's sums turned into FP64
 // once (block_moments), took another 4 us off a call.
@@ -1386,8 +1386,10 @@ __global__ void __launch_bounds__(256) k_stats_partial(const float *__restrict__
     Shifted2 m;
     const int64_t step = static_cast<int64_t>(gridDim.x) * blockDim.x;
     constexpr int U = 16;
+    int group = 0;
     for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += U * step) {
         float v[U];
+        if (++group % 64 == 0) m.flush();  // at most 1024 samples in FP32 sums
         const int left = static_cast<int>(min(static_cast<int64_t>(U), (n - i + step - 1) / step));
 #pragma unroll
         for (int k = 0; k < U; ++k)
