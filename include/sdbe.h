@@ -428,11 +428,14 @@ int sdbe_vdif_headers(void *frames, int64_t n_pkts, int64_t pol_stride_bytes, ui
  * P P^T solve and projection in FP64 (the systems are ill-conditioned).
  * 2 <= ntap <= 8; spec_c64 8-byte aligned.  The prototype compiles its
  * solve out (#if 0); this restates the method it sets up.  Uses handle
- * scratch of nblock*(12 + 8*ntap)*32768 bytes (up to 4096 blocks; the factor
- * of the solve is kept there for later calls of the same taps, and formed by
- * the call that first needs it; above, nblock*(4 + 8*ntap)*32768, formed as
- * the solve goes), allocated when a call needs
- * more than any earlier one (that growth synchronizes the device). */
+ * scratch of nblock*(12 + 8*ntap)*32768 bytes, grown by doubling (which
+ * synchronizes the device) up to 4096 blocks; the factor of the solve is kept
+ * there for later calls of the same taps, and formed by the call that first
+ * needs it, which waits for its stream.  Above 4096 blocks, or where there is
+ * no memory for that, the factor is formed as the solve goes, in
+ * nblock*(4 + 8*ntap)*32768 bytes.  A call can be captured into a CUDA graph
+ * after one of the same taps and at least as many blocks; the graph is valid
+ * until a call of other taps or of more blocks than any before. */
 int sdbe_inverse_pfb(sdbe_resampler *h, const void *spec_c64, int64_t nblock, int32_t ntap, float *out,
                      void *stream);
 

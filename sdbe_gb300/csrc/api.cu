@@ -79,6 +79,8 @@ void free_all(sdbe_resampler *h) {
     cudaFree(h->reform_dev);
     cudaFree(h->ipfb_tab);
     cudaFree(h->ipfb_y);
+    cudaFree(h->ipfb_fac);
+    cudaFree(h->ipfb_v);
     cudaFree(h->ipfb_scr);
     cudaFree(h->wring);
     cudaFree(h->wpart);

@@ -66,12 +66,15 @@ struct sdbe_resampler {
     sdbe_reform_state *reform_dev = nullptr;                // kernel's output state
     double *ipfb_tab = nullptr;   // inverse PFB: [3][ntap][32768] band of P P^T, P taps, taps over the middle one (FP64)
     int ipfb_ntap = 0;
-    uint8_t *ipfb_y = nullptr;    // inverse PFB scratch, grown to the largest call: with a kept factor the
-                                  // substituted values [nblock][32768] f64, then y [nblock][32768] f32
+    uint8_t *ipfb_y = nullptr;    // inverse PFB scratch, grown to the largest call: y [nblock][32768] f32
     int64_t ipfb_y_bytes = 0;
-    uint8_t *ipfb_scr = nullptr;  // factors [nblock][ntap][32768] f64
+    uint8_t *ipfb_fac = nullptr;  // the kept factor [rows][ntap][32768] f64, and the substituted values
+    int64_t ipfb_fac_bytes = 0;   // of calls that use it, [nblock][32768] f64
+    uint8_t *ipfb_v = nullptr;
+    int64_t ipfb_v_bytes = 0;
+    int64_t ipfb_rows = 0;        // rows of ipfb_fac that are formed (of ipfb_ntap taps)
+    uint8_t *ipfb_scr = nullptr;  // calls without it: factors [nblock][ntap][32768] f64
     int64_t ipfb_scr_bytes = 0;
-    int64_t ipfb_rows = 0;        // rows of the kept factor in ipfb_scr (of ipfb_ntap taps)
     uint8_t *pol_scr = nullptr;   // group assembly on the device: state, result, bins, codes
     int64_t pol_scr_bytes = 0;
     int64_t ing_last_n = 0;       // packets of the last sdbe_ingest batch (their flags in ing_accept)

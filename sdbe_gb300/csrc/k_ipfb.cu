@@ -25,9 +25,11 @@
 // a warp here) bound the solve, and forming the factor anew was two thirds of
 // them, so the handle keeps it, as it keeps the window's table: k_ipfb_factor
 // forms it once for the largest call so far (up to kPlanBlocks rows), and
-// k_ipfb_apply does the two substitutions.
+// k_ipfb_apply does the two substitutions.  Calls of more blocks, or without room
+// for it, form the factor as they go.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <type_traits>
 #include <vector>
@@ -390,6 +392,34 @@ cudaError_t with_taps(int ntap, F f) {
     }
 }
 
+// Room for at least `need` bytes, `want` if there is so much; a larger buffer
+// replaces the old one after all work on the device.
+bool make_room(uint8_t **buf, int64_t *cap, int64_t want, int64_t need) {
+    if (*cap >= need) return true;
+    if (*buf && cudaDeviceSynchronize() != cudaSuccess) return false;
+    cudaFree(*buf);
+    *buf = nullptr;
+    *cap = 0;
+    for (const int64_t bytes : {want > need ? want : need, need}) {
+        if (cudaMalloc(buf, static_cast<size_t>(bytes)) == cudaSuccess) {
+            *cap = bytes;
+            return true;
+        }
+        cudaGetLastError();
+        *buf = nullptr;
+    }
+    return false;
+}
+
+void drop_factor(sdbe_resampler *h) {
+    if (h->ipfb_fac || h->ipfb_v) cudaDeviceSynchronize();
+    cudaFree(h->ipfb_fac);
+    cudaFree(h->ipfb_v);
+    h->ipfb_fac = h->ipfb_v = nullptr;
+    h->ipfb_fac_bytes = h->ipfb_v_bytes = 0;
+    h->ipfb_rows = 0;
+}
+
 }  // namespace
 }  // namespace sdbe
 
@@ -405,46 +435,69 @@ extern "C" int sdbe_inverse_pfb(sdbe_resampler *h, const void *spec_c64, int64_t
     if (!g.ok) return fail(h, SDBE_ERR_CUDA, "cudaSetDevice failed");
     if (int rc = check_status(h)) return rc;
     cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : h->stream;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    SDBE_CK(h, cudaStreamIsCapturing(st, &cap));
+    const bool capturing = cap != cudaStreamCaptureStatusNone;
+    constexpr int64_t kRowF = kNA * static_cast<int64_t>(sizeof(float)), kRowD = 2 * kRowF;
     if (h->ipfb_ntap != ntap) {
         const std::vector<double> tab = ipfb_table(ntap);
-        if (h->ipfb_tab) {
-            SDBE_CK(h, cudaDeviceSynchronize());
-            cudaFree(h->ipfb_tab);
-            h->ipfb_tab = nullptr;
-            h->ipfb_ntap = 0;
-        }
+        if (h->ipfb_tab) SDBE_CK(h, cudaDeviceSynchronize());
+        h->ipfb_ntap = 0;
         h->ipfb_rows = 0;
-        SDBE_CK(h, cudaMalloc(&h->ipfb_tab, (tab.size() + static_cast<size_t>(ntap) * kNA) * sizeof(double)));
+        if (!h->ipfb_tab) SDBE_CK(h, cudaMalloc(&h->ipfb_tab, 3 * 8 * kRowD));  // of eight taps
         SDBE_CK(h, cudaMemcpyAsync(h->ipfb_tab, tab.data(), tab.size() * sizeof(double), cudaMemcpyHostToDevice, st));
         SDBE_CK(h, cudaStreamSynchronize(st));  // tab is freed on return
         h->ipfb_ntap = ntap;
     }
-    // scratch owned by the handle, grown to the largest call so far: the factor
-    // (or, above kPlanBlocks, the factor with the substituted values) and, with
-    // a kept factor, the substituted values, which first serve the tensor-core
-    // C2R as its paired spectra (n x 16384 complex)
-    const bool plan = nblock <= kPlanBlocks;
-    const int64_t v_bytes = plan ? nblock * kNA * static_cast<int64_t>(sizeof(double)) : 0;
-    if (int rc = grow(h, &h->ipfb_y, &h->ipfb_y_bytes, v_bytes + nblock * kNA * static_cast<int64_t>(sizeof(float)),
-                      "the inverse PFB scratch"))
-        return rc;
-    const int64_t need = nblock * ntap * kNA * static_cast<int64_t>(sizeof(double));
-    if (h->ipfb_scr_bytes < need || !plan) h->ipfb_rows = 0;  // the kept factor goes
-    if (int rc = grow(h, &h->ipfb_scr, &h->ipfb_scr_bytes, need, "the inverse PFB scratch")) return rc;
-    float *y = reinterpret_cast<float *>(h->ipfb_y + v_bytes);
-    double *scr = reinterpret_cast<double *>(h->ipfb_scr), *v = reinterpret_cast<double *>(h->ipfb_y);
-    if (plan && h->ipfb_rows < nblock) {
-        SDBE_CK(h, cudaDeviceSynchronize());  // calls on other streams may still read the scratch
-        SDBE_CK(h, with_taps(ntap, [&](auto nt) { return launch_factor<decltype(nt)::value>(nblock, h->ipfb_tab, scr, st); }));
-        SDBE_CK(h, cudaStreamSynchronize(st));  // later calls, on any stream, find it complete
-        h->ipfb_rows = nblock;
+    // Scratch owned by the handle, grown to the largest call so far and by
+    // doubling.  What a captured call uses is replaced only where its y is (a
+    // larger call) or its table (other taps): the factor and the substituted
+    // values are laid out for as many rows as y has, and calls without the
+    // factor have scratch of their own.  Where memory is short, or the stream
+    // is being captured and there is no room yet, a call forms its factor as it
+    // goes, which takes 8 nblock rows less.
+    const int64_t have = h->ipfb_y_bytes / kRowF;
+    const int64_t twice = nblock > kPlanBlocks ? nblock : std::min(2 * have, kPlanBlocks);
+    bool room = make_room(&h->ipfb_y, &h->ipfb_y_bytes, twice * kRowF, nblock * kRowF);
+    if (!room) {
+        if (!capturing) drop_factor(h);
+        if (int rc = grow(h, &h->ipfb_y, &h->ipfb_y_bytes, nblock * kRowF, "the inverse PFB scratch")) return rc;
+    }
+    float *y = reinterpret_cast<float *>(h->ipfb_y);
+    const int64_t rows = std::min(h->ipfb_y_bytes / kRowF, kPlanBlocks);
+    bool plan = nblock <= kPlanBlocks;
+    if (plan && capturing) {
+        plan = h->ipfb_v_bytes >= nblock * kRowD && h->ipfb_fac_bytes >= nblock * ntap * kRowD;
+    } else if (plan) {
+        if (h->ipfb_fac_bytes < nblock * ntap * kRowD) h->ipfb_rows = 0;
+        plan = make_room(&h->ipfb_v, &h->ipfb_v_bytes, rows * kRowD, nblock * kRowD) &&
+               make_room(&h->ipfb_fac, &h->ipfb_fac_bytes, rows * ntap * kRowD, nblock * ntap * kRowD);
+        if (!plan) drop_factor(h);
+    }
+    double *fac = reinterpret_cast<double *>(h->ipfb_fac), *v = reinterpret_cast<double *>(h->ipfb_v);
+    if (!plan) {
+        const int64_t need = nblock * ntap * kRowD;
+        if (!make_room(&h->ipfb_scr, &h->ipfb_scr_bytes, need, need)) {
+            if (!capturing) drop_factor(h);
+            if (int rc = grow(h, &h->ipfb_scr, &h->ipfb_scr_bytes, need, "the inverse PFB scratch")) return rc;
+        }
+        fac = v = reinterpret_cast<double *>(h->ipfb_scr);
+    } else if (h->ipfb_rows < nblock) {
+        // rows formed before are formed again, with the same values
+        const int64_t form = capturing ? nblock
+                                       : std::max(nblock, std::min(2 * h->ipfb_rows, h->ipfb_fac_bytes / (ntap * kRowD)));
+        SDBE_CK(h, with_taps(ntap, [&](auto nt) { return launch_factor<decltype(nt)::value>(form, h->ipfb_tab, fac, st); }));
         h->launches += 1;
+        if (!capturing) {  // (a captured call forms its rows in each replay)
+            SDBE_CK(h, cudaStreamSynchronize(st));  // later calls, on any stream, find them complete
+            h->ipfb_rows = form;
+        }
     }
     cudaError_t e = cudaSuccess;
     if (h->cfg.precision != SDBE_PRECISION_FP32) {
         // the pseudo time stream on the tensor cores
         if (int rc = tc_c2r_spectra(h, static_cast<const float2 *>(spec_c64), kMA + 1, nblock,
-                                    reinterpret_cast<float2 *>(plan ? v : scr), y, st))
+                                    reinterpret_cast<float2 *>(v), y, st))
             return rc;
     } else {
         e = launch_r2dbe_c2r(spec_c64, kMA + 1, nblock, 0, y, h->tw, st);
@@ -452,8 +505,8 @@ extern "C" int sdbe_inverse_pfb(sdbe_resampler *h, const void *spec_c64, int64_t
     if (e == cudaSuccess)
         e = with_taps(ntap, [&](auto nt) {
             constexpr int NT = decltype(nt)::value;
-            return plan ? launch_apply<NT>(y, nblock, h->ipfb_tab, scr, v, out, st)
-                        : launch_solve<NT>(y, nblock, h->ipfb_tab, scr, out, st);
+            return plan ? launch_apply<NT>(y, nblock, h->ipfb_tab, fac, v, out, st)
+                        : launch_solve<NT>(y, nblock, h->ipfb_tab, fac, out, st);
         });
     if (e != cudaSuccess) return fail(h, SDBE_ERR_CUDA, std::string("inverse_pfb: ") + cudaGetErrorString(e));
     h->launches += 2;
