@@ -454,8 +454,8 @@ __device__ __forceinline__ void fwd_pass8(float2 *sm, const TabsB &T) {
 // z[j + 1144 r] (8 consecutive j per 8 lanes: 64-B segments) and writes its 16
 // outputs to slots 16*rho(j) + r, rho = digit reversal of j over (8, 11, 13);
 // every later butterfly reads and writes the same slots g*Ns*R + k + Ns*r
-// with twiddles W_{Ns*R}^{k r}, so passes need no staging.
-//
+// with twiddles W_{Ns*R}^{k r}, so passes need no staging.  R2C: see fwd_pass8.
+template <bool R2C>
 __device__ __forceinline__ void fft18304_from_global(float2 *sm, const float2 *__restrict__ z, const TabsB &T) {
     constexpr int NB1 = kMB / 16;  // 1144 = 143 groups of 8
     for (int h = threadIdx.x >> 4; h < 72; h += blockDim.x >> 4) {
@@ -485,7 +485,7 @@ __device__ __forceinline__ void fft18304_from_global(float2 *sm, const float2 *_
     __syncthreads();
     fwd_pass11(sm, T);
     __syncthreads();
-    fwd_pass8<false>(sm, T);
+    fwd_pass8<R2C, R2C>(sm, T);
     __syncthreads();
 }
 
@@ -565,6 +565,21 @@ __device__ __forceinline__ int c2r_slot(int t) {
 __device__ __forceinline__ int c2r_sub(int t) {
     const int w = t >> 6, s = (t >> 5) & 1;
     return w == 0 ? 8 * s : (s ? 16 - w : w);
+}
+
+// The inverse's first-pass inputs Z'[j], j = col + 512 r, of the window Y[j] =
+// X[skip + j], j = 0..16384, by the C2R pairing on the fly (no pass of its own),
+// with W_32768^-j = wc e^{2 pi i r/64} (wc per thread, the rest compile-time);
+// Im Y[0] and Im Y[16384] are dropped.  A warp's columns are 16 apart, one
+// padded row of `sm` each: both runs, up from Y[col] and down from
+// Y[16384 - col], are conflict-free.
+__device__ __forceinline__ void c2r_window(float2 *v, const float2 *sm, int skip, int col, float2 wc) {
+    const float2 *lo = sm + padb(skip + col);        // Y[col + 512 r] = lo[544 r]
+    const float2 *hi = sm + padb(skip + kMA - col);  // Y[16384 - col - 512 r] = hi[-544 r]
+    for_r(std::make_integer_sequence<int, 32>{}, [&](auto rc) {
+        constexpr int r = decltype(rc)::value;
+        v[r] = c2r_pre<0, r == 0 ? 1 : 0>(lo[544 * r], hi[-544 * r], col + 512 * r, c2r_tw_rn<r>(wc));
+    });
 }
 
 // The C2R 32768 input Z[col + 512 r], r < 32, from the bins Y[0..16384]
@@ -1007,24 +1022,10 @@ __global__ void __launch_bounds__(kNTB, 1) k_resample(const __grid_constant__ Se
                          : "memory");
         }
         wait(&P.pass4, k);
-        // The inverse's first pass loads Z'[j], j = col + 512 r, computed on the
-        // fly by the C2R pairing of the window Y[j] = X[skip + j], j = 0..16384
-        // (no pass of its own), with W_32768^-j = wc e^{2 pi i r/64} (wc per
-        // thread, the rest compile-time); Im Y[0] and Im Y[16384] are dropped.
-        // A warp's columns are 16 apart, one padded row of `sm` each: both
-        // runs, up from Y[col] and down from Y[16384 - col], are conflict-free.
-        auto zin = [&](float2 *v) {
-            const float2 *lo = sm + padb(skip + col);        // Y[col + 512 r] = lo[544 r]
-            const float2 *hi = sm + padb(skip + kMA - col);  // Y[16384 - col - 512 r] = hi[-544 r]
-            for_r(std::make_integer_sequence<int, 32>{}, [&](auto rc) {
-                constexpr int r = decltype(rc)::value;
-                v[r] = c2r_pre<0, r == 0 ? 1 : 0>(lo[544 * r], hi[-544 * r], col + 512 * r, c2r_tw_rn<r>(wc));
-            });
-        };
         auto inverse = [&](auto epi) {
             {
                 float2 v[32];
-                zin(v);
+                c2r_window(v, sm, skip, col, wc);
                 arrive(&P.taken);
                 dft<32, true>(v);
                 wait(&P.taken, k);  // every read of X ends before the first stores over it
@@ -1137,6 +1138,42 @@ __global__ void __launch_bounds__(kNTB, 1) k_resample(const __grid_constant__ Se
     if (tid == 0 && tc5::flag_set(&P.err)) S.status.raise();
 }
 
+// k_resample<2> for at most one chunk per CTA: nothing to overlap, so no
+// pipeline to set up (tensor memory, stages, barriers), block barriers between
+// the passes.  A call of 1 to 152 chunks takes 24.8 us (bound by the latency of
+// each pass, 16 warps an SM), 29 through the pipeline; from 153 on a CTA has a
+// second chunk and the pipeline's 45 us are the same as two rounds of this.
+__global__ void __launch_bounds__(kNTB, 1)
+    k_resample_once(const float *__restrict__ in, int skip, float *__restrict__ out, Twiddles tw) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    float2 *sm = reinterpret_cast<float2 *>(smem_raw);
+    float2 *tb = sm + kPadB;
+    TabsA TA = tabs_a_at(tb);
+    TabsB TB = tabs_b_at(tb, tw);
+    load_tabs_ab(TA, TB, tw);
+    const int sub = threadIdx.x >> 5, col = sub + 16 * (threadIdx.x & 31);
+    const float2 wc = conjf2(__ldg(tw.w32768 + col));  // W_32768^-col
+    fft18304_from_global<true>(sm, reinterpret_cast<const float2 *>(in + static_cast<int64_t>(blockIdx.x) * kNB), TB);
+    float2 v[32];
+    c2r_window(v, sm, skip, col, wc);
+    dft<32, true>(v);
+    __syncthreads();  // every read of X ends before the first stores over it
+    inv_store1(sm + kSub * sub, col, v);
+    __syncwarp();
+    inv_pass2(sm + kSub * sub, [&](float2 *u) {
+        float2 w[32];
+        pass2_twiddles(TA, w);
+#pragma unroll
+        for (int r = 1; r < 32; ++r) u[r] = cmulc(u[r], w[r]);
+    });
+    __syncthreads();
+    float2 *dst = reinterpret_cast<float2 *>(out + static_cast<int64_t>(blockIdx.x) * kNC);
+    inv_pass3<true>([&](int r) { return sm + kSub * r; }, last_tw(TA), [&](int jj, const float2 *u) {
+#pragma unroll
+        for (int r = 0; r < 16; ++r) dst[jj + 1024 * r] = u[r];
+    }, [] {});
+}
+
 // SwarmR2C alone: complex64 [n][18305] spectra (persistent over chunks).
 __global__ void __launch_bounds__(kNTB, 1)
     k_swarm_r2c(const float *__restrict__ in, int64_t n_chunks, float2 *__restrict__ out, Twiddles tw) {
@@ -1147,7 +1184,7 @@ __global__ void __launch_bounds__(kNTB, 1)
     load_tabs_b(TB, tw);
     for (int64_t c = blockIdx.x; c < n_chunks; c += gridDim.x) {
         __syncthreads();
-        fft18304_from_global(sm, reinterpret_cast<const float2 *>(in + c * kNB), TB);
+        fft18304_from_global<false>(sm, reinterpret_cast<const float2 *>(in + c * kNB), TB);
         float2 *dst = out + c * (kMB + 1);
         for (int q = threadIdx.x; q <= kMB; q += kNTB) dst[q] = r2c_bin(sm, q, __ldg(tw.w36608 + q));
     }
@@ -1458,6 +1495,8 @@ cudaError_t configure_fft_kernels() {
         return e;
     if ((e = cudaFuncSetAttribute(k_resample<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemPipeB))) != cudaSuccess)
         return e;
+    if ((e = cudaFuncSetAttribute(k_resample_once, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemB))) != cudaSuccess)
+        return e;
     if ((e = cudaFuncSetAttribute(k_swarm_r2c, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemB))) != cudaSuccess)
         return e;
     if ((e = cudaFuncSetAttribute(k_r2dbe_c2r, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemB))) != cudaSuccess)
@@ -1494,6 +1533,8 @@ cudaError_t launch_resample_segs(int mode, const SegsB &S, const Twiddles &tw, c
         k_resample<3><<<grid, kNTB, kSmemPipeB, st>>>(S, tw);
     else if (mode == 1)
         k_resample<1><<<grid, kNTB, kSmemPipeB, st>>>(S, tw);
+    else if (S.n == 1 && static_cast<int64_t>(grid) == S.n_items && S.s[0].n_chunks == S.n_items)
+        k_resample_once<<<grid, kNTB, kSmemB, st>>>(S.s[0].in, S.s[0].skip, S.s[0].o.fout, tw);
     else
         k_resample<2><<<grid, kNTB, kSmemPipeB, st>>>(S, tw);
     return cudaGetLastError();
