@@ -257,7 +257,7 @@ typedef struct sdbe_reform_state {
     int32_t tprev_sec, tprev_clk; /* last counted packet's timestamp (TPREV)                */
     int64_t bprev;                /* its B-count (BPREV; a 32-bit int in the reference)     */
     int64_t marked_invalid;       /* packets invalidated for a jump beyond 1000 frames      */
-    int64_t slow_tiles;           /* 1024-packet tiles counted one packet at a time         */
+    int64_t slow_tiles;           /* 1024-packet tiles with pairs that were stepped           */
     int64_t reserved;
 } sdbe_reform_state;
 int sdbe_reform_init(sdbe_reform_state *st);

@@ -63,7 +63,8 @@ struct sdbe_resampler {
     uint8_t *ing_hdr = nullptr;    // [n][3] header words (w0, w4, w5) read back for the policy
     int64_t ing_hdr_bytes = 0;
     sdbe_reform_state reform{-1, -1, -1, -1, -1, 0, 0, 0};  // 8pac batches: reform state
-    sdbe_reform_state *reform_dev = nullptr;                // kernel's output state
+    uint8_t *reform_dev = nullptr;                          // kernel's output state, the check's findings
+    int64_t reform_dev_bytes = 0;
     double *ipfb_tab = nullptr;   // inverse PFB: [3][ntap][32768] band of P P^T, P taps, taps over the middle one (FP64)
     int ipfb_ntap = 0;
     uint8_t *ipfb_y = nullptr;    // inverse PFB scratch, grown to the largest call: y [nblock][32768] f32

@@ -197,10 +197,12 @@ int sdbe_ingest(sdbe_resampler *h, const void *packets, int64_t n_packets, void 
             }
             rc = grow(h, &h->ing_batch, &h->ing_batch_bytes, n_pk * kPktBytes, "ingest batch");
             if (rc) return rc;
-            if (!h->reform_dev) SDBE_CK(h, cudaMalloc(&h->reform_dev, kReformScratch));
+            rc = grow(h, &h->reform_dev, &h->reform_dev_bytes, reform_scratch(n_pk), "reform scratch");
+            if (rc) return rc;
+            sdbe_reform_state *reform_out = reinterpret_cast<sdbe_reform_state *>(h->reform_dev);
             SDBE_CK(h, launch_unpack_8pac(src, n_packets, h->ing_batch, st));
-            SDBE_CK(h, launch_beng_reform(h->ing_batch, n_pk, h->reform, h->reform_dev, hdr, st));
-            SDBE_CK(h, cudaMemcpyAsync(&reform, h->reform_dev, sizeof(reform), cudaMemcpyDeviceToHost, st));
+            SDBE_CK(h, launch_beng_reform(h->ing_batch, n_pk, h->reform, reform_out, hdr, st));
+            SDBE_CK(h, cudaMemcpyAsync(&reform, reform_out, sizeof(reform), cudaMemcpyDeviceToHost, st));
             h->launches += 2;
             dev_pkts = h->ing_batch;
         } else {

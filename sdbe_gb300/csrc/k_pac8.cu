@@ -64,18 +64,23 @@ __global__ void __launch_bounds__(256) k_unpack_8pac(const uint8_t *__restrict__
 // its predecessor have clk < 286e6 and lie a whole number k of frames apart
 // with |k| <= 1000, stepping returns exactly k (each step adds 262144 clocks
 // to the absolute time and lands on the other timestamp), so the counts are
-// BPREV plus a prefix sum: computed with block scans.  Any other tile (jitter,
-// corrupt clocks, jumps beyond the cap) is walked by one thread with the
-// stepping itself, bounded by the cap, so results match the reference in all
-// cases.
+// BPREV plus a prefix sum: computed with block scans.  Any other pair (jitter,
+// corrupt clocks) is stepped by its own thread, bounded by the cap.  A packet
+// beyond the cap becomes invalid, which changes its successor's predecessor:
+// such a tile is summed by one thread, which steps that pair anew.  So results
+// match the reference in all cases.  (With one thread stepping every pair of a
+// tile with jitter, 2048 packets took 218 us; 44 now, 155 with a jump.)
 //
-// Walking the tiles one after another takes 4.7 us a tile, most of it latency
-// (1353 us for the 292,864 packets of a group).  The usual batch is regular
+// Walking the tiles one after another takes 3.9 us a tile, most of it latency
+// (1122 us for the 292,864 packets of a group).  The usual batch is regular
 // throughout, and then each count is simply BPREV plus the B-frames from TPREV
 // to the packet's own timestamp: k_reform_check looks at every pair of
-// neighbouring valid packets, all tiles at once, and k_reform_apply rewrites
-// the headers; the walk runs only if a pair was irregular (or the batch is
-// shorter than kReformWalk packets, where three more launches cost more).
+// neighbouring valid packets, all tiles at once, and k_beng_reform then
+// rewrites the headers a tile per CTA; one CTA walks only if a pair was
+// irregular (or the batch is shorter than kReformWalk packets, where the other
+// launch costs as much as two tiles).  Whole calls by the walk /
+// with the check: 4096 packets 46.0 / 44.4 us, 8192 59.2 / 44.2, a group 1188 /
+// 143; the check costs an irregular batch 12 us.
 // ---------------------------------------------------------------------------
 struct Ts {
     int32_t sec, clk;
@@ -164,13 +169,14 @@ struct SumOp {
     __device__ long long operator()(long long a, long long b) const { return a + b; }
 };
 
-// What k_reform_check found: whether the walk is needed, and the timestamps of
-// the batch's first and last valid packets.
+// What k_reform_check found besides the tiles with irregular pairs (a byte
+// each, behind this): the timestamps of the batch's first and last valid
+// packets, if there are none of those.
 struct ReformInfo {
-    int irregular, reserved;
     Ts first, last;
 };
-constexpr int64_t kReformWalk = 2 * kReformThreads;
+constexpr int64_t kReformWalk = 4 * kReformThreads;
+__host__ __device__ constexpr int64_t reform_tiles(int64_t n) { return (n + kReformThreads - 1) / kReformThreads; }
 
 // Whole frames from p to ts within the stepping cap, both clocks in range.
 __device__ __forceinline__ bool regular_step(Ts p, Ts ts) {
@@ -185,6 +191,7 @@ __device__ __forceinline__ bool regular_step(Ts p, Ts ts) {
 // (over 1024 invalid packets in a row) the batch counts as irregular.
 __global__ void __launch_bounds__(kReformThreads) k_reform_check(const uint8_t *__restrict__ pkts, int64_t n,
                                                                  sdbe_reform_state in, ReformInfo *info) {
+    uint8_t *bad = reinterpret_cast<uint8_t *>(info + 1);
     __shared__ Ts s_ts[kReformThreads];
     __shared__ int s_pv[kReformThreads];
     __shared__ int s_scan_i[32];
@@ -229,13 +236,13 @@ __global__ void __launch_bounds__(kReformThreads) k_reform_check(const uint8_t *
     // the batch's first and last valid packets lie in its first and last tiles
     if (tid == 0 && last < 0 && (base == 0 || base + kReformThreads >= n)) ok = false;
     if (base + kReformThreads >= n && tid == last) info->last = ts;
-    if (__syncthreads_or(!ok) && tid == 0) info->irregular = 1;
+    const int irregular = __syncthreads_or(!ok);
+    if (tid == 0) bad[blockIdx.x] = irregular != 0;
 }
 
-__global__ void __launch_bounds__(256) k_reform_apply(uint8_t *__restrict__ pkts, int64_t n, sdbe_reform_state in,
-                                                      sdbe_reform_state *out, uint32_t *__restrict__ hdr,
-                                                      const ReformInfo *__restrict__ info) {
-    if (info->irregular) return;
+// This CTA's tile of a batch that is regular throughout.
+__device__ __forceinline__ void reform_tile(uint8_t *pkts, int64_t n, const sdbe_reform_state &in,
+                                            sdbe_reform_state *out, uint32_t *hdr, const ReformInfo *info) {
     const bool unset = in.t0_sec == -1 && in.t0_clk == -1;
     const Ts p = unset ? info->first : Ts{in.tprev_sec, in.tprev_clk};
     const long long bprev = unset ? 0 : in.bprev;
@@ -243,7 +250,7 @@ __global__ void __launch_bounds__(256) k_reform_apply(uint8_t *__restrict__ pkts
         const long long d = (static_cast<long long>(ts.sec - p.sec) * kClkPerSec + (ts.clk - p.clk)) / kBframeClk;
         return static_cast<int32_t>(static_cast<uint32_t>(static_cast<unsigned long long>(bprev + d)));
     };
-    const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    const int64_t i = static_cast<int64_t>(blockIdx.x) * kReformThreads + threadIdx.x;
     if (i < n) {
         uint32_t *w = reinterpret_cast<uint32_t *>(pkts + i * kPktBytes);
         const uint32_t w0 = w[0], w5 = w[5];
@@ -271,10 +278,20 @@ __global__ void __launch_bounds__(kReformThreads) k_beng_reform(uint8_t *__restr
                                                                 sdbe_reform_state in, sdbe_reform_state *out,
                                                                 uint32_t *__restrict__ hdr,
                                                                 const ReformInfo *__restrict__ info) {
-    if (info != nullptr && info->irregular == 0) return;  // k_reform_apply has done it
+    if (info != nullptr) {
+        const uint8_t *bad = reinterpret_cast<const uint8_t *>(info + 1);
+        bool irregular = false;
+        for (int64_t t = threadIdx.x; t < reform_tiles(n); t += kReformThreads) irregular |= bad[t] != 0;
+        if (!__syncthreads_or(irregular)) {
+            reform_tile(pkts, n, in, out, hdr, info);
+            return;
+        }
+        if (blockIdx.x > 0) return;
+    }
     __shared__ sdbe_reform_state s;
     __shared__ Ts s_ts[kReformThreads];
     __shared__ int s_pv[kReformThreads];
+    __shared__ int32_t s_off[kReformThreads];
     __shared__ int s_first;
     __shared__ int s_scan_i[32];
     __shared__ long long s_scan_l[32];
@@ -311,11 +328,21 @@ __global__ void __launch_bounds__(kReformThreads) k_beng_reform(uint8_t *__restr
         long long d = 0;
         if (valid) {
             const long long delta = static_cast<long long>(ts.sec - p.sec) * kClkPerSec + (ts.clk - p.clk);
-            ok = ts.clk < kClkPerSec && p.clk < kClkPerSec && ts.clk >= 0 && p.clk >= 0 &&
-                 delta % kBframeClk == 0 && delta <= kMaxOffset * kBframeClk && -delta <= kMaxOffset * kBframeClk;
+            const long long apart = delta < 0 ? -delta : delta;
+            const bool clocks = ts.clk < kClkPerSec && p.clk < kClkPerSec && ts.clk >= 0 && p.clk >= 0;
+            ok = clocks && delta % kBframeClk == 0 && apart <= kMaxOffset * kBframeClk;
             d = delta / kBframeClk;
+            // an irregular pair is stepped by its own thread, unless it is surely
+            // beyond the cap (which a pair that compares equal never is)
+            if (!ok)
+                d = clocks && apart > (kMaxOffset + 2) * kBframeClk && ts_compare(p, ts) != 0 ? kMaxOffset + 1
+                                                                                             : ts_offset(p, ts);
         }
-        const bool slow = __syncthreads_or(valid && !ok) != 0;
+        // A valid packet's predecessor is the valid one before it, unless that
+        // lies beyond the cap and becomes invalid: only then the tile is counted
+        // packet by packet.
+        const bool stepped = __syncthreads_or(valid && !ok) != 0;
+        const bool slow = stepped && __syncthreads_or(valid && (d > kMaxOffset || -d > kMaxOffset)) != 0;
         if (!slow) {
             const long long sum = block_scan_inclusive<long long>(valid ? d : 0, s_scan_l, SumOp(), 0);
             const int32_t off = static_cast<int32_t>(static_cast<uint32_t>(static_cast<unsigned long long>(s.bprev + sum)));
@@ -326,27 +353,41 @@ __global__ void __launch_bounds__(kReformThreads) k_beng_reform(uint8_t *__restr
                 s.tprev_clk = ts.clk;
                 s.bprev = off;
             }
-        } else if (tid == 0) {
-            const int64_t end = n - base < kReformThreads ? n - base : kReformThreads;
-            for (int64_t j = 0; j < end; ++j) {
-                uint32_t *wj = reinterpret_cast<uint32_t *>(pkts + (base + j) * kPktBytes);
-                if (wj[0] >> 31) continue;
-                const uint32_t w5j = wj[5];
-                const Ts now = read_ts(wj[4], w5j);
-                int32_t off = static_cast<int32_t>(ts_offset(Ts{s.tprev_sec, s.tprev_clk}, now));
-                if (off > kMaxOffset || off < -kMaxOffset) {
-                    wj[0] |= 0x80000000u;
-                    off = -1;
-                    s.marked_invalid += 1;
-                } else {
-                    off = static_cast<int32_t>(static_cast<uint32_t>(static_cast<unsigned long long>(off + s.bprev)));
-                    s.tprev_sec = now.sec;
-                    s.tprev_clk = now.clk;
-                    s.bprev = off;
+            if (stepped && tid == 0) s.slow_tiles += 1;
+        } else {
+            s_off[tid] = static_cast<int32_t>(d);  // |d| <= kMaxOffset + 1
+            __syncthreads();
+            if (tid == 0) {
+                const int end = static_cast<int>(n - base < kReformThreads ? n - base : kReformThreads);
+                Ts prev{s.tprev_sec, s.tprev_clk};
+                long long bprev = s.bprev;
+                bool marked = false;  // the valid packet before
+                for (int j = 0; j < end; ++j) {
+                    if (s_pv[j] != j) continue;
+                    const Ts now = s_ts[j];
+                    int32_t off = marked ? static_cast<int32_t>(ts_offset(prev, now)) : s_off[j];
+                    marked = off > kMaxOffset || off < -kMaxOffset;
+                    if (marked) {
+                        s_pv[j] = -1;
+                        off = -1;
+                        s.marked_invalid += 1;
+                    } else {
+                        off = static_cast<int32_t>(static_cast<uint32_t>(static_cast<unsigned long long>(off + bprev)));
+                        prev = now;
+                        bprev = off;
+                    }
+                    s_off[j] = off;
                 }
-                write_old_header(wj, w5j, off);
+                s.tprev_sec = prev.sec;
+                s.tprev_clk = prev.clk;
+                s.bprev = bprev;
+                s.slow_tiles += 1;
             }
-            s.slow_tiles += 1;
+            __syncthreads();
+            if (valid) {
+                if (s_pv[tid] != tid) w[0] |= 0x80000000u;
+                write_old_header(w, w5, s_off[tid]);
+            }
         }
         __syncthreads();
         if (hdr != nullptr && i < n) {
@@ -377,23 +418,25 @@ cudaError_t launch_unpack_8pac(const void *src, int64_t n_units, void *dst, cuda
     return cudaGetLastError();
 }
 
-// out_dev: kReformScratch bytes.
+// Device bytes: the state after a batch of n packets, then the check's findings.
+int64_t reform_scratch(int64_t n) {
+    return static_cast<int64_t>(sizeof(sdbe_reform_state) + sizeof(ReformInfo)) + reform_tiles(n);
+}
+
+// out_dev: reform_scratch(n) bytes.
 cudaError_t launch_beng_reform(void *pkts, int64_t n, const sdbe_reform_state &in, sdbe_reform_state *out_dev,
                                uint32_t *hdr, cudaStream_t st) {
-    static_assert(sizeof(sdbe_reform_state) + sizeof(ReformInfo) <= kReformScratch, "reform scratch");
     uint8_t *p = static_cast<uint8_t *>(pkts);
     ReformInfo *info = nullptr;
+    unsigned grid = 1;
     if (n >= kReformWalk) {
         info = reinterpret_cast<ReformInfo *>(out_dev + 1);
-        cudaError_t e = cudaMemsetAsync(info, 0, sizeof(ReformInfo), st);
-        if (e != cudaSuccess) return e;
-        k_reform_check<<<static_cast<unsigned>((n + kReformThreads - 1) / kReformThreads), kReformThreads, 0, st>>>(
-            p, n, in, info);
-        k_reform_apply<<<static_cast<unsigned>((n + 255) / 256), 256, 0, st>>>(p, n, in, out_dev, hdr, info);
-        e = cudaGetLastError();
+        grid = static_cast<unsigned>(reform_tiles(n));
+        k_reform_check<<<grid, kReformThreads, 0, st>>>(p, n, in, info);
+        const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
-    k_beng_reform<<<1, kReformThreads, 0, st>>>(p, n, in, out_dev, hdr, info);
+    k_beng_reform<<<grid, kReformThreads, 0, st>>>(p, n, in, out_dev, hdr, info);
     return cudaGetLastError();
 }
 
@@ -432,7 +475,7 @@ int sdbe_beng_reform(sdbe_reform_state *st, void *pkts, int64_t n_pkts, void *st
     if (n_pkts == 0) return SDBE_OK;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     void *scr = nullptr;  // this thread's reusable scratch: the call waits for its stream below
-    SDBE_CK(nullptr, thread_scratch(kReformScratch, &scr));
+    SDBE_CK(nullptr, thread_scratch(static_cast<size_t>(reform_scratch(n_pkts)), &scr));
     sdbe_reform_state *dev = static_cast<sdbe_reform_state *>(scr);
     cudaError_t e = launch_beng_reform(pkts, n_pkts, *st, dev, nullptr, s);
     sdbe_reform_state out{};
