@@ -523,7 +523,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_fft(const __grid_constant_
         // every FP16 half below 2^14 without a pass for the maximum.  TMEM is
         // read GC chunks of 8 columns per wait.
         const int k1 = quarter * 32 + lane;
-        constexpr int GC = G::RES ? 4 : 1;  // one chunk where registers are short
+        constexpr int GC = G::RES ? 2 : 1;  // four spill 284 bytes: 22 us a C2R of 48 blocks for 18
         static_assert(GC == 1 || NCH % (GC * kTcParts) == 0, "chunk groups");
         constexpr float s2 = 1.f / 256.f;
         const int rot = lane >> 3;  // = (k1 >> 3) & 3
