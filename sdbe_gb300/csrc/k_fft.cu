@@ -857,8 +857,8 @@ __global__ void __launch_bounds__(kNTB, 1) k_resample(const __grid_constant__ Se
     TabsB TB = tabs_b_at(tb, tw);
     __shared__ double red[64];
     __shared__ PipeB P;
-    // the forms with float output run a chunk or two per CTA as a rule
-    constexpr bool ROLL = MODE == 1 || MODE == 2;
+    // the first batch runs a chunk or two per CTA (6000 chunks of floats alone: 687 us rolled, 676 not)
+    constexpr bool ROLL = MODE == 1;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (tid == 0) {
         uint64_t *bars[6] = {&P.xfree, &P.pass2, &P.pass3, &P.pass4, &P.taken, &P.inv2};
@@ -1138,11 +1138,11 @@ __global__ void __launch_bounds__(kNTB, 1) k_resample(const __grid_constant__ Se
     if (tid == 0 && tc5::flag_set(&P.err)) S.status.raise();
 }
 
-// k_resample<2> for at most one chunk per CTA: nothing to overlap, so no
-// pipeline to set up (tensor memory, stages, barriers), block barriers between
-// the passes.  A call of 1 to 152 chunks takes 24.8 us (bound by the latency of
-// each pass, 16 warps an SM), 29 through the pipeline; from 153 on a CTA has a
-// second chunk and the pipeline's 45 us are the same as two rounds of this.
+// k_resample<2> for at most two chunks per SM, one CTA each: little to overlap,
+// so no pipeline to set up (tensor memory, stages, barriers), block barriers
+// between the passes.  A call of 1 to 152 chunks takes 24.8 us (bound by the
+// latency of each pass, 16 warps an SM), 29 through the pipeline, 153 to 304
+// take 42 to 43 (46 to 48), 456 would take 69.4 (68.3).
 __global__ void __launch_bounds__(kNTB, 1)
     k_resample_once(const float *__restrict__ in, int skip, float *__restrict__ out, Twiddles tw) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1533,8 +1533,8 @@ cudaError_t launch_resample_segs(int mode, const SegsB &S, const Twiddles &tw, c
         k_resample<3><<<grid, kNTB, kSmemPipeB, st>>>(S, tw);
     else if (mode == 1)
         k_resample<1><<<grid, kNTB, kSmemPipeB, st>>>(S, tw);
-    else if (S.n == 1 && static_cast<int64_t>(grid) == S.n_items && S.s[0].n_chunks == S.n_items)
-        k_resample_once<<<grid, kNTB, kSmemB, st>>>(S.s[0].in, S.s[0].skip, S.s[0].o.fout, tw);
+    else if (S.n == 1 && S.n_items <= 2 * static_cast<int64_t>(grid) && S.s[0].n_chunks == S.n_items)
+        k_resample_once<<<static_cast<unsigned>(S.n_items), kNTB, kSmemB, st>>>(S.s[0].in, S.s[0].skip, S.s[0].o.fout, tw);
     else
         k_resample<2><<<grid, kNTB, kSmemPipeB, st>>>(S, tw);
     return cudaGetLastError();
