@@ -101,6 +101,42 @@ def test_without_the_kept_factor(R, ntap):
         assert _close(_capture(r, S, ntap)(), ref)
 
 
+@pytest.fixture(scope="module")
+def solver(R):
+    """A handle whose captured calls of up to 8 spectra form their factor as they go."""
+    with R(max_frames=1) as r:
+        _inv(r, _spectra(4097, 5), 4)
+        yield r
+
+
+@pytest.mark.parametrize("scale", [0.0, 1e-45, 1e-43, 1e-41, 1e-39, 1e-36, 1.0, 1e30, 2e34, 1e36, "inf row", "nan row"])
+def test_values_converted_by_parts(R, solver, scale):
+    """Time samples and blocks that are zero, denormal, ordinary, large, beyond
+    FP32's range or not finite: the kept factor's integer conversions against
+    FP64 instructions.  Tolerance: FP32's last place, and 1e-10 of the RMS for the
+    other order of the FP64 operations."""
+    import torch
+
+    S = _spectra(8, 77)
+    if isinstance(scale, str):
+        S[3, 100] = float(scale.split()[0])
+    else:
+        S = (S.to(torch.complex128) * scale).to(torch.complex64)
+    with R(max_frames=1) as r:
+        got = _inv(r, S, 4).double()
+    ref = _capture(solver, S, 4)().double()
+    for test in (torch.isnan, torch.isposinf, torch.isneginf):
+        assert torch.equal(test(got), test(ref))
+    ok = torch.isfinite(ref)
+    if scale == 0.0:
+        assert not bool(got.any())
+    if not bool(ok.any()):
+        return
+    a, b = got[ok], ref[ok]
+    rms = float(b.pow(2).mean().sqrt()) if float(b.abs().max()) < 1e150 else float(b.abs().max())
+    assert bool(((a - b).abs() <= 2.0 ** -23 * b.abs() + 2.0 ** -149 + 1e-10 * rms).all())
+
+
 @pytest.mark.parametrize("nb", [4096, 4097])
 def test_longest_kept_and_shortest_formed_as_it_goes(R, nb):
     """The blocks' forward PFB gives the pseudo time stream again.  A residual
