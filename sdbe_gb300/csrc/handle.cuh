@@ -173,8 +173,10 @@ inline int64_t wave_len(const sdbe_resampler *h, int64_t wave, int64_t remaining
     int64_t nb = remaining < wave ? remaining : wave;
     // Payloads that leave for the host wave by wave: what the last wave ships
     // is not behind any compute, so the last waves shrink (a wave's copy takes
-    // about a sixth of its compute).  128 batches of 143 frames in host
-    // memory: 8178 -> 7073 us with the FFT pipelines, 7617 without this.
+    // about a sixth of its compute).  Calls on host buffers without / with
+    // this: 8 frames 543 / 529 us, 20 1242 / 1140, 60 3493 / 3054, 143 7510 /
+    // 6967, 300 no change.  (How fast host memory takes them differs from
+    // machine to machine; up to six batches the waves left are too short.)
     if (h->shipping && remaining <= wave && remaining > 6) nb = (3 * remaining + 3) / 4;
     if (h->cfg.threshold_mode == SDBE_THRESH_WINDOW) {
         const int64_t to_block = SDBE_THRESH_BLOCK - h->stream_batch % SDBE_THRESH_BLOCK;
