@@ -73,13 +73,14 @@ def test_stage_functions_report_it(N, stage, name):
 
     from sdbe_gb300 import Resampler
 
-    a, b = (torch.zeros(36608, device="cuda") for _ in range(2))
+    n = 2 * torch.cuda.get_device_properties(0).multi_processor_count + 1  # fewer chunks run without waits
+    a, b = (torch.zeros(n * 36608, device="cuda") for _ in range(2))
     with Resampler(max_frames=2) as rs:
         N.check(N.lib().sdbe_test_fft_timeout(rs.handle, stage), rs.handle)
         fn = getattr(N.lib(), name)
-        assert fn(rs.handle, a.data_ptr(), 1, b.data_ptr(), None) == N.OK
+        assert fn(rs.handle, a.data_ptr(), n, b.data_ptr(), None) == N.OK
         _timed_out(N, rs.sync)
-        assert fn(rs.handle, a.data_ptr(), 1, b.data_ptr(), None) == N.ERR_CUDA
+        assert fn(rs.handle, a.data_ptr(), n, b.data_ptr(), None) == N.ERR_CUDA
 
 
 @pytest.mark.parametrize("stage", [1, 2])
