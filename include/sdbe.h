@@ -381,7 +381,8 @@ int sdbe_r2dbe_c2r(sdbe_resampler *h, const void *in_c64, int64_t n_chunks, int3
 int sdbe_resample_chunks(sdbe_resampler *h, const float *in, int64_t n_chunks, float *out,
                          void *stream);
 
-/* summary_stats + transform_reduce (.cu:66-137,953-977) in FP64:
+/* summary_stats + transform_reduce (.cu:66-137,953-977), no further from exact
+ * sums than FP64 ones:
  * out[0] = mean (quantizeOffset), out[1] = sqrt(M2/(n-1)) (quantizeThreshold).
  * The sums are of the samples minus the first one, so a large common offset
  * does not cancel digits of the variance.  Uses scratch of the calling thread
